@@ -426,6 +426,29 @@ __device__ __forceinline__ bool compose_inverse(double P[6], const double d[6]) 
   return true;
 }
 
+// compose_inverse with one reciprocal of the determinant instead of six divisions (the FP64
+// results differ in their last bits).
+__device__ __forceinline__ bool compose_inverse_rcp(double P[6], const double d[6]) {
+  const double det = (1 + d[0]) * (1 + d[3]) - d[1] * d[2];
+  if (!(det != 0)) return false;
+  const double id = 1.0 / det;
+  const double t1 = (-d[0] - d[0] * d[3] + d[1] * d[2]) * id;
+  const double t2 = -d[1] * id;
+  const double t3 = -d[2] * id;
+  const double t4 = (-d[3] - d[0] * d[3] + d[1] * d[2]) * id;
+  const double t5 = (-d[4] - d[3] * d[4] + d[2] * d[5]) * id;
+  const double t6 = (-d[5] - d[0] * d[5] + d[1] * d[4]) * id;
+  const double a00 = 1 + P[0], a01 = P[2], a02 = P[4];
+  const double a10 = P[1], a11 = 1 + P[3], a12 = P[5];
+  P[0] = a00 * (1 + t1) + a01 * t2 - 1;
+  P[1] = a10 * (1 + t1) + a11 * t2;
+  P[2] = a00 * t3 + a01 * (1 + t4);
+  P[3] = a10 * t3 + a11 * (1 + t4) - 1;
+  P[4] = a00 * t5 + a01 * t6 + a02;
+  P[5] = a10 * t5 + a11 * t6 + a12;
+  return true;
+}
+
 // x = A^-1 b for an n x n (n <= 6) column-major system, Gaussian elimination with
 // partial pivoting in FP64 (mldivide's general path; a zero pivot yields Inf/NaN).
 __device__ inline void solve_small(int n, const double* Ain, const double* bin, double* x) {

@@ -657,16 +657,7 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
 // fast 6-DOF solve for subsets at the nominal window without a mask region
 // ================================================================================
 // The common case (uniform variant; quadtree subsets whose window holds no masked or zero
-// pixel) needs no flood fill, so a group of NW warps solves one subset with no shared image
-// buffer.  Every thread walks its share of the window pixels; the sums are warp shuffles
-// (FP32 per thread, FP64 across lanes) plus, for NW > 1, one fixed-order FP64 sum of the
-// NW warp totals behind a named barrier of the group, so every thread holds the same
-// totals and runs the same FP64 Gauss-Newton control redundantly: there is no other
-// barrier per iteration.  The gradients f_x, f_y are re-read from the L1-resident gradient
-// images each iteration.  The 6x6 inverse is a per-group [H | I] Gauss-Jordan elimination
-// without pivoting by the group's first warp (H is the symmetric positive semi-definite
-// Gauss-Newton Hessian; a zero pivot propagates Inf/NaN as the reference's singular solve
-// does).
+// pixel) needs no flood fill, so a group of NW warps solves one subset (icgn_tile.cuh).
 //
 // The main pass (NW = 1, queue 0) gives each subset at most warp_cap iterations (8 by
 // default; 6-12 measured within 1 % of each other on the stereo pass, 4 and 24 slower): the
@@ -713,602 +704,11 @@ __device__ __forceinline__ void group_sum(double (&v)[K], double* red, int gw, i
   group_bar<NW>(bar);
 }
 
-// The one-warp pass is latency-bound on its image reads: three CTAs per SM (24 warps, 80
-// registers with a few spills) measured 12 % faster than two (128 registers, no spills);
-// four (64 registers) spill too much.
-// Staging (STAGED): every group owns a shared-memory buffer of box_r x box_c floats (the
-// box of a TMA tensor map over the deformed image, column-major) and an mbarrier.  Before an
-// iteration it computes the tap footprint of the warped window (0-based image rows / columns
-// from the window's corners in the pixel loop's own FP32 arithmetic, one row / column of
-// margin) and, when that leaves the staged box, loads a new box whose first row is rounded
-// down to a 16-byte boundary (the TMA rule for the innermost coordinate).  The stencil then
-// reads shared memory with the same operations as the gather path, so values are
-// bit-identical.  An iteration whose footprint exceeds the box (a large deformation) gathers
-// from the image.  A wait that outlasts kTmaWaitCycles sets qcount[8] and the group gathers
-// from the image from then on.
-constexpr long long kTmaWaitCycles = 2000000000LL;  // ~1 s at the B200 clock
-constexpr size_t kStageBytesMax = 100 * 1024;       // staging buffers of one block: two blocks per SM
+}  // namespace aldic
 
-struct StageGeom {
-  int box_r, box_c;  // tensor-map box: rows (a multiple of 4) x columns
-  int buf_floats;    // floats per group buffer (a multiple of 32: 128-byte aligned buffers)
-};
+#include "icgn_tile.cuh"
 
-// Tap footprint (0-based image rows rlo..rhi, columns clo..chi) of the warped window of an
-// iteration: the window's corners in the pixel loop's own FP32 arithmetic, one row / column
-// of margin on each side (an interior pixel's floor() may differ from a corner's by one).
-__device__ __forceinline__ void tap_footprint(float p0, float p1, float p2, float p3, float f5, float f6, int half,
-                                              int br, int bc, int& rlo, int& rhi, int& clo, int& chi) {
-  float lxmin = 3.0e38f, lxmax = -3.0e38f, lymin = 3.0e38f, lymax = -3.0e38f;
-#pragma unroll
-  for (int cx = -1; cx <= 1; cx += 2)
-#pragma unroll
-    for (int cy = -1; cy <= 1; cy += 2) {
-      const float dxc = (float)(cx * half), dyc = (float)(cy * half);
-      const float lx = dxc + fmaf(p0, dxc, fmaf(p2, dyc, f5));
-      const float ly = dyc + fmaf(p3, dyc, fmaf(p1, dxc, f6));
-      lxmin = fminf(lxmin, lx);
-      lxmax = fmaxf(lxmax, lx);
-      lymin = fminf(lymin, ly);
-      lymax = fmaxf(lymax, ly);
-    }
-  rlo = br + (int)floorf(lxmin) - 1;
-  rhi = br + (int)floorf(lxmax) + 4;
-  clo = bc + (int)floorf(lymin) - 1;
-  chi = bc + (int)floorf(lymax) + 4;
-}
-
-// Issue the TMA load of the box that covers a footprint (its first row rounded down to a
-// 16-byte boundary) into the group's buffer; false when the footprint does not fit a box.  The
-// caller has no load in flight into this buffer.  Every thread of the group calls it.
-template <int NW>
-__device__ __forceinline__ bool stage_issue(const CUtensorMap& tmap, float* tile, int BR, int BC, int rlo, int rhi,
-                                            int clo, int chi, uint64_t& bar_mem, int bar, int gt, int& tr0,
-                                            int& tc0) {
-  const int nr0 = rlo - (((rlo % 4) + 4) % 4);
-  if (!(rhi - nr0 < BR && chi - clo < BC)) return false;
-  fence_proxy_async_shared();  // this thread's reads of the old box before the copy writes
-  group_bar<NW>(bar);
-  if (gt == 0) {
-    mbar_arrive_expect_tx(&bar_mem, (uint32_t)(BR * BC * 4));
-    tma_load_2d(tile, &tmap, nr0, clo, &bar_mem);
-  }
-  tr0 = nr0;
-  tc0 = clo;
-  return true;
-}
-
-// Wait for the group's load in flight (every thread polls; the outcome is agreed by the group).
-// On time-out the group gathers from the image from then on and flags qcount[8].
-template <int NW>
-__device__ __forceinline__ void stage_wait(bool& pending, bool& tile_ok, bool& broken, uint32_t& phase,
-                                           uint64_t& bar_mem, int& ok_mem, int bar, int gt, int* qcount) {
-  bool ok = mbar_wait(&bar_mem, phase, kTmaWaitCycles);
-  if (NW == 1) {
-    ok = __all_sync(0xffffffffu, ok);
-  } else {
-    if (gt == 0) ok_mem = 1;
-    group_bar<NW>(bar);
-    if (!ok) ok_mem = 0;
-    group_bar<NW>(bar);
-    ok = ok_mem != 0;
-  }
-  if (ok) {
-    phase ^= 1;
-    pending = false;
-    tile_ok = true;
-  } else {
-    broken = true;  // the copy may still land: the buffer is never reused
-    tile_ok = false;
-    if (gt == 0) atomicOr(qcount + 8, 1);
-  }
-}
-
-template <int NW, bool SLOW, bool STAGED>
-__global__ void __launch_bounds__(kWT, STAGED ? 2 : (NW == 1 ? 3 : 2))
-    icgn_group_kernel(IcgnArgs a, const __grid_constant__ CUtensorMap tmap, StageGeom geo) {
-  constexpr int NG = kWT / (32 * NW);  // subset groups per CTA
-  constexpr int GT = 32 * NW;          // threads per group
-  extern __shared__ __align__(128) float s_tiles[];
-  __shared__ __align__(8) uint64_t s_bar[NG];
-  __shared__ int s_ok[NG];
-  __shared__ double s_aug[NG][72];     // 6 x 12 row-major [H | I] -> [I | H^-1]
-  __shared__ double s_ab[NG][12];      // A (0..5), B (6..11)
-  __shared__ double s_h[NG][21];       // packed upper triangle by rows
-  __shared__ double s_fac[NG][6];      // elimination factors of the current pivot column
-  __shared__ double s_red[NG][NW * 21];
-  const int lane = threadIdx.x & 31, grp = threadIdx.x / GT, gw = (threadIdx.x % GT) >> 5;
-  const int gt = threadIdx.x % GT, bar = 1 + grp;
-  double* aug = s_aug[grp];
-  double* AB = s_ab[grp];
-  double* red = s_red[grp];
-  const FrameDev& fr = a.fr;
-  const bool quad = (a.variant == 1);
-  const bool epi = (a.variant == 2);
-  const bool want_fg = epi || a.zncc != nullptr;  // sum f g: the epipolar ZNSSD, or the ZNCC
-  __shared__ int s_qi[NG];
-  const int count = a.qcount[SLOW ? 1 : 0];
-  const int gM = fr.M - 6;
-  int* next = a.qcount + (SLOW ? 3 : 2);  // work counter of this pass (zeroed with the queues)
-  // staging state of the group (replicated in its threads)
-  // the buffers start at the first 128-byte boundary of the dynamic shared memory (the launch
-  // allocates 128 bytes more than the buffers need)
-  float* tile = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(s_tiles) + 127) & ~uintptr_t(127)) +
-                (STAGED ? grp * geo.buf_floats : 0);
-  const int BR = geo.box_r, BC = geo.box_c;
-  int tr0 = 0, tc0 = 0;
-  bool tile_ok = false, pending = false, broken = false;
-  uint32_t phase = 0;
-  if (STAGED) {
-    if (gt == 0) {
-      mbar_init(&s_bar[grp], 1);
-      fence_barrier_init();
-    }
-    group_bar<NW>(bar);
-  }
-  while (true) {
-    // the group's next queue entry (dynamic: slow subsets do not pile up on one group)
-    int qi = 0;
-    if (gt == 0) qi = atomicAdd(next, 1);
-    if (NW == 1) {
-      qi = __shfl_sync(0xffffffffu, qi, 0);
-    } else {
-      if (gt == 0) s_qi[grp] = qi;
-      group_bar<NW>(bar);
-      qi = s_qi[grp];
-    }
-    if (qi >= count) {
-      // a copy in flight (a prefetch never used, or one that outlasted its wait) must land
-      // before the block's shared memory is released
-      if (STAGED && (pending || broken)) mbar_wait(&s_bar[grp], phase, kTmaWaitCycles);
-      break;
-    }
-    const int* q = a.queue + 3 * ((SLOW ? a.n : 0) + qi);
-    if (SLOW && q[2] != kSlowSubset) {
-      group_bar<NW>(bar);
-      continue;
-    }
-    const long long t = q[0];
-    const int w = q[1];
-    const int W1 = w + 1, npx = W1 * W1, half = w / 2;
-    double x0 = a.coords[t], y0 = a.coords[a.n + t];
-    if (quad) {
-      x0 = mround(x0);
-      y0 = mround(y0);
-    }
-    const int r0 = (int)x0 - half - 1, c0 = (int)y0 - half - 1;
-    const int q_nt = GT / W1, r_nt = GT % W1;
-    if constexpr (STAGED) {
-      // prefetch the first iteration's box (P = [0 0 0 0 U0], or the carried state) so the
-      // load overlaps the set-up sums
-      if (!broken && !pending) {
-        double Pp[6] = {0.0, 0.0, 0.0, 0.0, epi ? 0.0 : a.U0[2 * t], epi ? 0.0 : a.U0[2 * t + 1]};
-        if (a.F0 && !epi)
-          for (int k = 0; k < 4; ++k) Pp[k] = a.F0[4 * t + k];
-        if (SLOW && a.carry)
-          for (int k = 0; k < 6; ++k) Pp[k] = a.carry[8 * t + k];
-        const double m5 = mround(Pp[4]), m6 = mround(Pp[5]);
-        if (isfinite(m5) && isfinite(m6) && fabs(m5) < 1e6 && fabs(m6) < 1e6) {
-          int rlo, rhi, clo, chi;
-          tap_footprint((float)Pp[0], (float)Pp[1], (float)Pp[2], (float)Pp[3], (float)(Pp[4] - m5),
-                        (float)(Pp[5] - m6), half, (int)(x0 + m5) - 2, (int)(y0 + m6) - 2, rlo, rhi, clo, chi);
-          const bool covered = tile_ok && rlo >= tr0 && rhi < tr0 + BR && clo >= tc0 && chi < tc0 + BC;
-          if (!covered && stage_issue<NW>(tmap, tile, BR, BC, rlo, rhi, clo, chi, s_bar[grp], bar, gt, tr0, tc0)) {
-            pending = true;
-            tile_ok = false;
-          }
-        }
-      }
-    }
-    // ---- set-up sums, FP64 per lane (J = gradient x integer offset is exact in FP64), in two
-    //      passes over the window to bound the live accumulators ----
-    double meanf, bf, sabsf;
-    {
-      double jf[6], jb[6], fs = 0.0, fs2 = 0.0, fab = 0.0;
-      float fn = 0.f;
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        jf[k] = 0.0;
-        jb[k] = 0.0;
-      }
-      int aa = gt % W1, bb = gt / W1;
-      for (int p = gt; p < npx; p += GT) {
-        const int k = (r0 + aa) + (c0 + bb) * fr.M;
-        const int kg = (r0 + aa - a.crop) + (c0 + bb - a.crop) * gM;
-        const float ff = fr.ref[k];  // a quadtree subset here has no masked pixel
-        const double f = ff, gxv = fr.gx[kg], gyv = fr.gy[kg];
-        const double dx = (double)(aa - half), dy = (double)(bb - half);
-        const double J[6] = {gxv * dx, gyv * dx, gxv * dy, gyv * dy, gxv, gyv};
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-          jf[i] = fma(J[i], f, jf[i]);
-          jb[i] += J[i];
-        }
-        if (!quad || fabsf(ff) > 1e-10f) {
-          fs += f;
-          fs2 = fma(f, f, fs2);
-          fn += 1.f;
-        }
-        fab += fabs(f);
-        aa += r_nt;
-        bb += q_nt;
-        if (aa >= W1) {
-          aa -= W1;
-          bb += 1;
-        }
-      }
-      {
-        double v[4] = {fs, fs2, (double)fn, fab};
-        group_sum<NW, 4>(v, red, gw, lane, bar);
-        sabsf = v[3];
-        if (v[2] > 0) {
-          meanf = v[0] / v[2];
-          bf = sqrt(fmax(v[1] - v[0] * v[0] / v[2], 0.0));
-        } else {
-          meanf = ALDIC_NAN;
-          bf = ALDIC_NAN;
-        }
-      }
-      {
-        double v[12];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          v[k] = jb[k];
-          v[6 + k] = jf[k];
-        }
-        group_sum<NW, 12>(v, red, gw, lane, bar);
-        if (gt < 6) {
-#pragma unroll
-          for (int k = 0; k < 6; ++k)
-            if (gt == k) {
-              AB[6 + k] = v[k];
-              AB[k] = (v[6 + k] - meanf * v[k]) / bf;
-            }
-        }
-      }
-    }
-    {
-      double h[21];
-#pragma unroll
-      for (int k = 0; k < 21; ++k) h[k] = 0.0;
-      int aa = gt % W1, bb = gt / W1;
-      for (int p = gt; p < npx; p += GT) {
-        const int kg = (r0 + aa - a.crop) + (c0 + bb - a.crop) * gM;
-        const double gxv = fr.gx[kg], gyv = fr.gy[kg];
-        const double dx = (double)(aa - half), dy = (double)(bb - half);
-        const double J[6] = {gxv * dx, gyv * dx, gxv * dy, gyv * dy, gxv, gyv};
-#pragma unroll
-        for (int i = 0; i < 6; ++i)
-#pragma unroll
-          for (int j = i; j < 6; ++j) {
-            const int m = i * 6 - i * (i - 1) / 2 + (j - i);  // packed upper triangle by rows
-            h[m] = fma(J[i], J[j], h[m]);
-          }
-        aa += r_nt;
-        bb += q_nt;
-        if (aa >= W1) {
-          aa -= W1;
-          bb += 1;
-        }
-      }
-      group_sum<NW, 21>(h, red, gw, lane, bar);
-      if (gt < 21) {
-#pragma unroll
-        for (int k = 0; k < 21; ++k)
-          if (gt == k) s_h[grp][k] = h[k];
-      }
-    }
-    group_bar<NW>(bar);
-    if (gw == 0) {
-      for (int e = lane; e < 72; e += 32) {
-        const int i = e / 12, j = e % 12;
-        double val;
-        if (j < 6) {
-          const int r = i < j ? i : j, cc = i < j ? j : i;  // packed upper-triangle index of (r, cc)
-          val = s_h[grp][r * 6 - r * (r - 1) / 2 + (cc - r)];
-        } else {
-          val = (j - 6 == i) ? 1.0 : 0.0;
-        }
-        aug[e] = val;
-      }
-      __syncwarp();
-      for (int k = 0; k < 6; ++k) {
-        // partial pivoting: the row (>= k) with the largest |entry| in column k, first one on
-        // ties (the mldivide of funICGN.m:288 pivots as well)
-        double best = lane >= k && lane < 6 ? fabs(aug[lane * 12 + k]) : -1.0;
-        int piv = lane;
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) {
-          const double ob = __shfl_down_sync(0xffffffffu, best, o);
-          const int op = __shfl_down_sync(0xffffffffu, piv, o);
-          if (lane + o < 8 && (ob > best || (ob == best && op < piv))) {
-            best = ob;
-            piv = op;
-          }
-        }
-        piv = __shfl_sync(0xffffffffu, piv, 0);
-        if (piv != k && lane < 12) {
-          const double tk = aug[k * 12 + lane];
-          aug[k * 12 + lane] = aug[piv * 12 + lane];
-          aug[piv * 12 + lane] = tk;
-        }
-        __syncwarp();
-        if (lane < 6) s_fac[grp][lane] = aug[lane * 12 + k];
-        const double pv = aug[k * 12 + k];
-        __syncwarp();
-        if (lane < 12) aug[k * 12 + lane] /= pv;
-        __syncwarp();
-        for (int e = lane; e < 72; e += 32) {
-          const int i = e / 12, j = e % 12;
-          if (i != k) aug[e] -= s_fac[grp][i] * aug[k * 12 + j];
-        }
-        __syncwarp();
-      }
-    }
-    group_bar<NW>(bar);
-    // ---- Gauss-Newton iterations (control replicated in every thread) ----
-    const double trH = s_h[grp][0] + s_h[grp][6] + s_h[grp][11] + s_h[grp][15] + s_h[grp][18] + s_h[grp][20];
-    double P[6] = {0.0, 0.0, 0.0, 0.0, epi ? 0.0 : a.U0[2 * t], epi ? 0.0 : a.U0[2 * t + 1]};
-    if (a.F0 && !epi)
-      for (int k = 0; k < 4; ++k) P[k] = a.F0[4 * t + k];  // a gradient initial guess (learned)
-    double normNew = 1.0, normAbs = 1.0, normInit = 0.0, znssd = ALDIC_NAN;
-    int step = 0, status = 0, requeue = -1;
-    if (SLOW && a.carry) {  // continue from where the warp pass stopped: P, the first norm, the step
-      const double* cs = a.carry + 8 * t;
-#pragma unroll
-      for (int k = 0; k < 6; ++k) P[k] = cs[k];
-      normInit = cs[6];
-      step = (int)cs[7];
-    }
-    while (step <= a.max_iter && normNew > a.tol && normAbs > a.tol) {
-      if (!SLOW && step >= a.warp_cap) {
-        // a long trajectory: FP32 rounding accumulates along it, so it is re-solved in FP64
-        // from its initial guess (or, for the epipolar score, continued by the multi-warp pass)
-        requeue = (a.slow_fp64 && !epi) ? kToFp64 : kSlowSubset;
-        break;
-      }
-      step += 1;
-      if (warped_oob(fr, P, x0, y0, half, half)) {
-        normNew = 1e6;
-        break;
-      }
-      const double n5 = mround(P[4]), n6 = mround(P[5]);
-      const float p0 = (float)P[0], p1 = (float)P[1], p2 = (float)P[2], p3 = (float)P[3];
-      const float f5 = (float)(P[4] - n5), f6 = (float)(P[5] - n6);
-      const int br = (int)(x0 + n5) - 2, bc = (int)(y0 + n6) - 2;
-      bool use_tile = false;
-      if constexpr (STAGED) {
-        if (!broken) {
-          int rlo, rhi, clo, chi;
-          tap_footprint(p0, p1, p2, p3, f5, f6, half, br, bc, rlo, rhi, clo, chi);
-          const bool covered = rlo >= tr0 && rhi < tr0 + BR && clo >= tc0 && chi < tc0 + BC;
-          if (!(covered && (tile_ok || pending))) {
-            // the staged (or prefetched) box misses this footprint: load the one that covers it
-            if (pending) stage_wait<NW>(pending, tile_ok, broken, phase, s_bar[grp], s_ok[grp], bar, gt, a.qcount);
-            tile_ok = false;
-            if (!broken && stage_issue<NW>(tmap, tile, BR, BC, rlo, rhi, clo, chi, s_bar[grp], bar, gt, tr0, tc0))
-              pending = true;
-          }
-          if (pending) stage_wait<NW>(pending, tile_ok, broken, phase, s_bar[grp], s_ok[grp], bar, gt, a.qcount);
-          use_tile = tile_ok && !broken;
-        }
-      }
-      // per-lane sums of the pixel pairs (p, p + GT) in packed FP32 with Kahan compensation
-      // (s + k is the compensated total; 3 extra packed operations per term), a last unpaired
-      // pixel alone; the lane totals go to FP64 before the cross-lane sums
-      double v[11];
-      {
-        float2 C2[6], K2[6], S12 = make_float2(0.f, 0.f), KS1 = make_float2(0.f, 0.f);
-        float2 S22 = make_float2(0.f, 0.f), KS2 = make_float2(0.f, 0.f), fg2 = make_float2(0.f, 0.f);
-        float S1 = 0.f, kS1 = 0.f, S2 = 0.f, kS2 = 0.f, ns = 0.f, nz = 0.f;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          C2[k] = make_float2(0.f, 0.f);
-          K2[k] = make_float2(0.f, 0.f);
-        }
-        const float2 pp0 = make_float2(p0, p0), pp1 = make_float2(p1, p1), pp2 = make_float2(p2, p2);
-        const float2 pp3 = make_float2(p3, p3), ff5 = make_float2(f5, f5), ff6 = make_float2(f6, f6);
-        int aa = gt % W1, bb = gt / W1;
-        int p = gt;
-        for (; p + GT < npx; p += 2 * GT) {
-          int ab = aa + r_nt, bbb = bb + q_nt;
-          if (ab >= W1) {
-            ab -= W1;
-            bbb += 1;
-          }
-          const float2 dx = make_float2((float)(aa - half), (float)(ab - half));
-          const float2 dy = make_float2((float)(bb - half), (float)(bbb - half));
-          const float2 lx = fadd2(dx, ffma2(pp0, dx, ffma2(pp2, dy, ff5)));
-          const float2 ly = fadd2(dy, ffma2(pp3, dy, ffma2(pp1, dx, ff6)));
-          const float ixa = floorf(lx.x), ixb = floorf(lx.y), iya = floorf(ly.x), iyb = floorf(ly.y);
-          const float2 tr = make_float2(lx.x - ixa, lx.y - ixb), tc = make_float2(ly.x - iya, ly.y - iyb);
-          float2 g;
-          if (STAGED && use_tile) {
-            const int oa = (br + (int)ixa - tr0) + (bc + (int)iya - tc0) * BR;
-            const int ob = (br + (int)ixb - tr0) + (bc + (int)iyb - tc0) * BR;
-            g = stencil16_x2_tile(tile, BR, oa, ob, tr, tc);
-          } else {
-            const int ia = (br + (int)ixa) + (bc + (int)iya) * fr.M, ib = (br + (int)ixb) + (bc + (int)iyb) * fr.M;
-            g = stencil16_x2(fr.def, fr.M, ia, ib, tr, tc);
-          }
-          const int ka = (r0 + aa - a.crop) + (c0 + bb - a.crop) * gM;
-          const int kb = (r0 + ab - a.crop) + (c0 + bbb - a.crop) * gM;
-          const float2 ag = fmul2(make_float2(fr.gx[ka], fr.gx[kb]), g);
-          const float2 bg = fmul2(make_float2(fr.gy[ka], fr.gy[kb]), g);
-          kahan2(C2[0], K2[0], ffma2(ag, dx, K2[0]));
-          kahan2(C2[1], K2[1], ffma2(bg, dx, K2[1]));
-          kahan2(C2[2], K2[2], ffma2(ag, dy, K2[2]));
-          kahan2(C2[3], K2[3], ffma2(bg, dy, K2[3]));
-          kahan2(C2[4], K2[4], fadd2(ag, K2[4]));
-          kahan2(C2[5], K2[5], fadd2(bg, K2[5]));
-          if (!quad) {
-            kahan2(S12, KS1, fadd2(g, KS1));
-            kahan2(S22, KS2, ffma2(g, g, KS2));
-          } else {
-            if (fabsf(g.x) > 1e-10f) {
-              kahan1(S1, kS1, g.x + kS1);
-              kahan1(S2, kS2, fmaf(g.x, g.x, kS2));
-              ns += 1.f;
-            }
-            if (fabsf(g.y) > 1e-10f) {
-              kahan1(S1, kS1, g.y + kS1);
-              kahan1(S2, kS2, fmaf(g.y, g.y, kS2));
-              ns += 1.f;
-            }
-            nz += (g.x == 0.f ? 1.f : 0.f) + (g.y == 0.f ? 1.f : 0.f);
-          }
-          if (want_fg)
-            fg2 = ffma2(make_float2(fr.ref[(r0 + aa) + (c0 + bb) * fr.M], fr.ref[(r0 + ab) + (c0 + bbb) * fr.M]), g,
-                        fg2);
-          aa = ab + r_nt;
-          bb = bbb + q_nt;
-          if (aa >= W1) {
-            aa -= W1;
-            bb += 1;
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < 6; ++k)
-          v[k] = ((double)C2[k].x + (double)K2[k].x) + ((double)C2[k].y + (double)K2[k].y);
-        if (!quad) {
-          v[6] = ((double)S12.x + (double)KS1.x) + ((double)S12.y + (double)KS1.y);
-          v[7] = ((double)S22.x + (double)KS2.x) + ((double)S22.y + (double)KS2.y);
-          ns = (float)((npx - gt + GT - 1) / GT);  // pixels of this thread
-        } else {
-          v[6] = (double)S1 + (double)kS1;
-          v[7] = (double)S2 + (double)kS2;
-        }
-        v[10] = (double)fg2.x + (double)fg2.y;
-        if (p < npx) {  // the last, unpaired pixel
-          const float dx = (float)(aa - half), dy = (float)(bb - half);
-          const float lx = dx + fmaf(p0, dx, fmaf(p2, dy, f5));
-          const float ly = dy + fmaf(p3, dy, fmaf(p1, dx, f6));
-          const float ix = floorf(lx), iy = floorf(ly);
-          const float g = (STAGED && use_tile)
-                              ? stencil16_tile(tile, BR, (br + (int)ix - tr0) + (bc + (int)iy - tc0) * BR, lx - ix,
-                                               ly - iy)
-                              : stencil16(fr.def, fr.M, br + (int)ix, bc + (int)iy, lx - ix, ly - iy);
-          const int kg = (r0 + aa - a.crop) + (c0 + bb - a.crop) * gM;
-          const float ag = fr.gx[kg] * g, bg = fr.gy[kg] * g;
-          v[0] += (double)(ag * dx);
-          v[1] += (double)(bg * dx);
-          v[2] += (double)(ag * dy);
-          v[3] += (double)(bg * dy);
-          v[4] += (double)ag;
-          v[5] += (double)bg;
-          if (quad) {
-            if (fabsf(g) > 1e-10f) {
-              v[6] += (double)g;
-              v[7] += (double)g * (double)g;
-              ns += 1.f;
-            }
-            if (g == 0.f) nz += 1.f;
-          } else {
-            v[6] += (double)g;
-            v[7] += (double)g * (double)g;
-          }
-          if (want_fg) v[10] += (double)fr.ref[(r0 + aa) + (c0 + bb) * fr.M] * (double)g;
-        }
-        v[8] = ns;
-        v[9] = nz;
-      }
-      group_sum<NW, 11>(v, red, gw, lane, bar);
-      if (v[9] > 0) {  // exact zero in g: the g-region flood fill is needed
-        requeue = 0;
-        break;
-      }
-      double meang, bgn;
-      if (v[8] > 0) {
-        meang = v[6] / v[8];
-        bgn = sqrt(fmax(v[7] - v[6] * v[6] / v[8], 0.0));
-      } else {
-        meang = ALDIC_NAN;
-        bgn = ALDIC_NAN;
-      }
-      if (want_fg) znssd = 2.0 - 2.0 * (v[10] - meanf * v[6]) / (bf * bgn);
-      double b[6];
-      const double ibgn = 1.0 / bgn;  // one FP64 division per iteration instead of six
-#pragma unroll
-      for (int k = 0; k < 6; ++k) b[k] = bf * (AB[k] - (v[k] - meang * AB[6 + k]) * ibgn);
-      double dP[6];
-#pragma unroll
-      for (int i = 0; i < 6; ++i) {
-        double acc = 0;
-#pragma unroll
-        for (int j = 0; j < 6; ++j) acc += aug[i * 12 + 6 + j] * b[j];
-        dP[i] = -acc;
-      }
-      double nn = 0;
-#pragma unroll
-      for (int i = 0; i < 6; ++i) nn += b[i] * b[i];
-      normNew = sqrt(nn);
-      normAbs = normNew;
-      if (step == 1) normInit = normNew;
-      if (normInit > a.tol) normNew = normNew / normInit;
-      else normNew = 0.0;
-      if (!epi && too_close_to_call(normNew, normAbs, normInit, a.tol, a.band,
-                                    fp32_noise(a.noise, step, bf, bgn, trH, v[7], v[8]))) {
-        requeue = kToFp64;  // the FP64 pass re-solves this subset from its initial guess
-        break;
-      }
-      if (!(normNew < a.tol || normAbs < a.tol)) {
-        if (!compose_inverse(P, dP)) {
-          step = a.max_iter + 1000;
-          status = 1;
-        } else if (epi) {
-          P[4] = 0.0;
-          P[5] = 0.0;
-        }
-      }
-    }
-    if (gt == 0) {
-      if (requeue == kToFp64) {
-        push_fp64(a, t, w, 0);  // unmasked, at the window this pass solved
-        if (SLOW) const_cast<int*>(q)[2] = kMovedSubset;
-        requeue = -2;
-      }
-      if (requeue == kSlowSubset && a.carry) {
-        double* cs = a.carry + 8 * t;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) cs[k] = P[k];
-        cs[6] = normInit;
-        cs[7] = (double)step;
-      }
-      if (requeue >= 0) {
-        // hand this subset to a later pass (they run after this kernel).  A queue-0
-        // subset is appended to queue 1 (at most one entry each: queue 1 never holds more
-        // than n); a queue-1 subset is re-flagged in place.
-        if (SLOW) {
-          const_cast<int*>(q)[2] = requeue;
-        } else {
-          const int pos = atomicAdd(&a.qcount[1], 1);
-          int* q1 = a.queue + 3 * ((long long)a.n + pos);
-          q1[0] = (int)t;
-          q1[1] = w;
-          q1[2] = requeue;
-        }
-      } else if (requeue == -1) {
-        if (status == 1) step -= 1000;
-        if (!(normNew < a.tol || normAbs < a.tol)) step = a.max_iter + 1;
-        if (isnan(normNew)) step = a.max_iter + 1;
-        if (quad && sabsf < 1e-6) step = a.max_iter + 3;
-        if (epi) {
-          a.znssd[t] = znssd;
-          if (a.conv) a.conv[t] = step;
-        } else {
-          a.conv[t] = step;
-          a.U[2 * t] = P[4];
-          a.U[2 * t + 1] = P[5];
-          for (int k = 0; k < 4; ++k) a.F[4 * t + k] = P[k];
-          if (want_fg) a.zncc[t] = 1.0 - 0.5 * znssd;
-          if (a.H)
-            for (int k = 0; k < 21; ++k) a.H[t + a.n * k] = s_h[grp][k];
-        }
-      }
-    }
-    group_bar<NW>(bar);
-  }
-}
+namespace aldic {
 
 // ================================================================================
 // Subpb1: classify + solve
@@ -1933,35 +1333,6 @@ __global__ void __launch_bounds__(kWT, 2) subpb1_group_kernel(Sub1Args a) {
   }
 }
 
-// Tensor map of a column-major FP32 image for the staging boxes (see tma.cuh).
-bool make_tmap_2d_f32(CUtensorMap* map, const float* base, int M, int N, int box_r, int box_c) {
-  using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess && fn)
-      encode = reinterpret_cast<EncodeFn>(fn);
-    else
-      cudaGetLastError();
-  });
-  if (!encode || !base || M < 1 || N < 1) return false;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ((size_t)M * sizeof(float)) % 16 != 0) return false;
-  if (box_r < 4 || box_r > 256 || box_r % 4 != 0 || box_c < 1 || box_c > 256) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)M, (cuuint64_t)N};
-  const cuuint64_t strides[1] = {(cuuint64_t)M * sizeof(float)};  // bytes between columns
-  const cuuint32_t box[2] = {(cuuint32_t)box_r, (cuuint32_t)box_c};
-  const cuuint32_t estride[2] = {1, 1};
-  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box,
-                            estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
-}
-
 int launch_icgn(const IcgnArgs& a, int wmax_enlarged, cudaStream_t st) {
   int launches = 0;
   // counts of buckets 0 and 1, the 2 work counters, the count of bucket 2, the staging flag
@@ -1973,49 +1344,14 @@ int launch_icgn(const IcgnArgs& a, int wmax_enlarged, cudaStream_t st) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  {  // nominal-window subsets without a mask region: one warp per subset, then the slow ones
-    // TMA staging of the deformed window when the tensor map can describe the image and the
-    // per-group boxes fit two blocks per SM; the gather path otherwise
-    StageGeom geo{0, 0, 0};
-    CUtensorMap tmap;
-    std::memset(&tmap, 0, sizeof(tmap));
-    bool staged = false;
-    if (a.staging) {
-      const int W1 = a.winsize + 1;
-      geo.box_r = (W1 + 14 + 3) / 4 * 4;  // footprint W1 + 5, alignment 3, 6 rows of deformation
-      geo.box_c = W1 + 11;                // footprint W1 + 5, 6 columns of deformation
-      geo.buf_floats = (geo.box_r * geo.box_c + 31) / 32 * 32;
-      const size_t bytes = (size_t)(kWT / 32) * geo.buf_floats * sizeof(float) + 128;
-      staged = geo.box_r <= 256 && geo.box_c <= 256 && bytes <= kStageBytesMax &&
-               make_tmap_2d_f32(&tmap, a.fr.def, a.fr.M, a.fr.N, geo.box_r, geo.box_c);
-    }
-    const int snw = a.slow_nw == 4 ? 4 : kSlowNW;
-    const size_t smem1 = staged ? (size_t)(kWT / 32) * geo.buf_floats * sizeof(float) + 128 : 0;
-    const size_t smem2 = staged ? (size_t)(kWT / (32 * snw)) * geo.buf_floats * sizeof(float) + 128 : 0;
-    auto k1 = staged ? icgn_group_kernel<1, false, true> : icgn_group_kernel<1, false, false>;
-    auto k2 = snw == 4 ? (staged ? icgn_group_kernel<4, true, true> : icgn_group_kernel<4, true, false>)
-                       : (staged ? icgn_group_kernel<kSlowNW, true, true> : icgn_group_kernel<kSlowNW, true, false>);
-    if (staged) {
-      cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
-      cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
-    }
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k1, kWT, smem1);
-    long long grid = (long long)sms * (per_sm < 1 ? 1 : per_sm);
-    const long long need = (a.n + 7) / 8;
-    if (grid > need) grid = need;
-    k1<<<(unsigned)grid, kWT, smem1, st>>>(a, tmap, geo);
-    ++launches;
-    if (!a.slow_fp64 || a.variant == 2) {  // the FP32 multi-warp pass continues the slow subsets
-      per_sm = 1;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k2, kWT, smem2);
-      grid = (long long)sms * (per_sm < 1 ? 1 : per_sm);
-      const long long need_slow = (a.n + kWT / (32 * snw) - 1) / (kWT / (32 * snw));
-      if (grid > need_slow) grid = need_slow;
-      k2<<<(unsigned)grid, kWT, smem2, st>>>(a, tmap, geo);
-      ++launches;
-    }
-  }
+  // nominal-window subsets without a mask region: one warp per subset, then the slow ones.
+  // Windows of which at least 4 CTAs' buffers fit an SM are staged in shared memory;
+  // ALDIC_OPT_STAGING stages every window whose buffers fit.
+  const TileGeom geo = tile_geometry(a.winsize + 1, a.staging ? 1 : 4);
+  launches += launch_icgn_tile<1, false>(a, geo, sms, st);
+  if (!a.slow_fp64 || a.variant == 2)  // the FP32 multi-warp pass continues the slow subsets
+    launches += a.slow_nw == 4 ? launch_icgn_tile<4, true>(a, geo, sms, st)
+                               : launch_icgn_tile<kSlowNW, true>(a, geo, sms, st);
   {  // enlarged / masked subsets, and those handed over by the fast kernel
     const size_t smem = icgn_smem_bytes(wmax_enlarged);
     cudaFuncSetAttribute(icgn_solve_kernel<false, kNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
