@@ -87,17 +87,28 @@ __device__ __forceinline__ f32x2_t pstencil(typename Taps<SMEM>::Ptr qa, typenam
   f32x2_t wr[4], wc[4];
   pweights(tr, wr);
   pweights(tc, wc);
-  f32x2_t acc = 0;
+  // taps by scalar FMAs on the weights' halves: pairing the loaded taps costs more moves than the
+  // packed form saves issue slots
+  float ra[4], rb[4], ca[4], cb[4], aa = 0.f, ab = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    upk(wr[k], ra[k], rb[k]);
+    upk(wc[k], ca[k], cb[k]);
+  }
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    f32x2_t col = pmul(wr[0], pk(T::ld(qa), T::ld(qb)));
+    float va = ra[0] * T::ld(qa), vb = rb[0] * T::ld(qb);
 #pragma unroll
-    for (int r = 1; r < 4; ++r) col = pfma(wr[r], pk(T::ld(T::at(qa, r)), T::ld(T::at(qb, r))), col);
-    acc = pfma(wc[c], col, acc);
+    for (int r = 1; r < 4; ++r) {
+      va = fmaf(ra[r], T::ld(T::at(qa, r)), va);
+      vb = fmaf(rb[r], T::ld(T::at(qb, r)), vb);
+    }
+    aa = fmaf(ca[c], va, aa);
+    ab = fmaf(cb[c], vb, ab);
     qa = T::at(qa, pitch);
     qb = T::at(qb, pitch);
   }
-  return acc;
+  return pk(aa, ab);
 }
 // stencil16 of common.cuh
 template <bool SMEM>
