@@ -54,37 +54,29 @@ __device__ __forceinline__ float stencil16(const float* __restrict__ img, int M,
 // decision was too close to call.  All 16 taps in bounds.
 __device__ __forceinline__ double stencil16_ref64(const float* __restrict__ img, int M, int r0, int c0, double tr,
                                                   double tc) {
-  constexpr int K[4][4] = {{0, 1, 0, 0}, {11, 1, -15, 3}, {19, -39, 25, -5}, {-3, 8, -8, 3}};
-  constexpr double sgn[4] = {1.0, -1.0, 1.0, 1.0};
+  // The scales depend on (i, j) only through the classes {0}, {1, 2}, {3} of each index, so the
+  // four powers of tr are combined once per class of j (R0, R1, R3) and column.
   const double s356 = (double)(3.0f / 56.0f), s17 = (double)(1.0f / 7.0f);
   const double s9 = (double)((1.0f / 3136.0f) * 9.0f), s3392 = (double)(3.0f / 392.0f);
   const double s149 = (double)(1.0f / 49.0f);
-  const double one[4] = {1.0, s356, s356, s17};
   const float* p = img + (size_t)r0 + (size_t)c0 * M;
-  double rowc[4][4];  // rowc[i][c] = sum_r K_i[r] Q[r][c]
+  const double tr2 = tr * tr, tr3 = tr2 * tr, tc2 = tc * tc, tc3 = tc2 * tc;
+  double R0 = 0.0, R1[4], R3[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const double q0 = __ldg(p + (size_t)c * M), q1 = __ldg(p + (size_t)c * M + 1);
     const double q2 = __ldg(p + (size_t)c * M + 2), q3 = __ldg(p + (size_t)c * M + 3);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) rowc[i][c] = ((K[i][0] * q0 + K[i][1] * q1) + K[i][2] * q2) + K[i][3] * q3;
+    const double k1 = ((11 * q0 + q1) + -15 * q2) + 3 * q3, k2 = ((19 * q0 + -39 * q1) + 25 * q2) + -5 * q3;
+    const double k3 = ((-3 * q0 + 8 * q1) + -8 * q2) + 3 * q3;
+    const double e12 = fma(k2, tr2, -(k1 * tr)), e3 = k3 * tr3;
+    if (c == 1) R0 = fma(s17, e3, fma(s356, e12, q1));
+    R1[c] = fma(s3392, e3, fma(s9, e12, s356 * q1));
+    R3[c] = fma(s149, e3, fma(s3392, e12, s17 * q1));
   }
-  const double pr[4] = {1.0, tr, tr * tr, tr * tr * tr};
-  const double pc[4] = {1.0, tc, tc * tc, tc * tc * tc};
-  double val = 0.0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const double t = ((K[j][0] * rowc[i][0] + K[j][1] * rowc[i][1]) + K[j][2] * rowc[i][2]) + K[j][3] * rowc[i][3];
-      double s;
-      if (i == 0 || j == 0) s = (i == 0) ? one[j] : one[i];
-      else if (i == 3 && j == 3) s = s149;
-      else if (i == 3 || j == 3) s = s3392;
-      else s = s9;
-      val += sgn[i] * sgn[j] * s * t * pr[i] * pc[j];
-    }
-  return val;
+  const double j1 = ((11 * R1[0] + R1[1]) + -15 * R1[2]) + 3 * R1[3];
+  const double j2 = ((19 * R1[0] + -39 * R1[1]) + 25 * R1[2]) + -5 * R1[3];
+  const double j3 = ((-3 * R3[0] + 8 * R3[1]) + -8 * R3[2]) + 3 * R3[3];
+  return fma(j3, tc3, fma(j2, tc2, fma(-j1, tc, R0)));
 }
 
 // Clamped version for arbitrary points (the MEX clamps taps to the image edge,
@@ -352,47 +344,131 @@ __device__ __forceinline__ void block_sum_dyn(double (&v)[K], double* scratch, d
 }
 
 // ---------------------------------------------------------------------------------
-// bwselect: connected component of `on` pixels (rows x cols, column-major, u8) that
-// contains the 0-based seed (sr, sc), 4- or 8-connected, into `lab` (u8).  Iterated
-// in-place propagation until no pixel changes; bounded by rows*cols sweeps (every
-// productive sweep adds at least one pixel).  All threads of the block must call it.
+// Bit columns: a mask of up to 128 rows as two 64-bit words per column (word 2 c + r / 64, bit
+// r % 64).  The flood fills of the solvers run on them: one warp, lanes = columns; a fill along a
+// column is six doubling steps on the words, a fill across columns five doubling steps of warp
+// shuffles, alternated until nothing changes (a few rounds for the regions met, where a sweep
+// over pixels needs as many rounds as the region is wide).
 // ---------------------------------------------------------------------------------
-__device__ inline void flood_select(const uint8_t* on, uint8_t* lab, int rows, int cols, int sr, int sc, int conn,
-                             int* flag) {
-  const int npx = rows * cols;
-  for (int p = threadIdx.x; p < npx; p += blockDim.x) lab[p] = 0;
-  __syncthreads();
-  const bool seed_ok = sr >= 0 && sr < rows && sc >= 0 && sc < cols && on[sr + sc * rows];
-  if (!seed_ok) {
-    __syncthreads();
-    return;
-  }
-  if (threadIdx.x == 0) lab[sr + sc * rows] = 1;
-  __syncthreads();
-  for (int sweep = 0; sweep < npx; ++sweep) {
-    int changed = 0;
-    for (int p = threadIdx.x; p < npx; p += blockDim.x) {
-      if (lab[p] || !on[p]) continue;
-      const int r = p % rows, c = p / rows;
-      bool hit = false;
-      if (r > 0 && lab[p - 1]) hit = true;
-      if (r + 1 < rows && lab[p + 1]) hit = true;
-      if (c > 0 && lab[p - rows]) hit = true;
-      if (c + 1 < cols && lab[p + rows]) hit = true;
-      if (!hit && conn == 8) {
-        if (r > 0 && c > 0 && lab[p - 1 - rows]) hit = true;
-        if (r + 1 < rows && c > 0 && lab[p + 1 - rows]) hit = true;
-        if (r > 0 && c + 1 < cols && lab[p - 1 + rows]) hit = true;
-        if (r + 1 < rows && c + 1 < cols && lab[p + 1 + rows]) hit = true;
-      }
-      if (hit) {
-        lab[p] = 1;
-        changed = 1;
-      }
+__device__ __forceinline__ bool bit_at(const uint64_t* m, int r, int c) { return (m[2 * c + (r >> 6)] >> (r & 63)) & 1; }
+
+// m = on(r, c) over rows x cols (rows <= 128); all nt threads of the block call it.
+template <class On>
+__device__ __forceinline__ void build_bits(uint64_t* m, int rows, int cols, int nt, On on) {
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < cols; c += nt >> 5) {
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int r = 32 * k + lane;
+      w[k] = 32 * k < rows ? __ballot_sync(0xffffffffu, r < rows && on(r, c)) : 0u;
     }
-    if (!__syncthreads_or(changed)) break;
+    if (lane < 2) m[2 * c + lane] = lane ? (uint64_t)w[3] << 32 | w[2] : (uint64_t)w[1] << 32 | w[0];
   }
-  (void)flag;
+}
+
+// Whether every bit of rows x cols is set (uniform over the block).
+__device__ __forceinline__ bool bits_full(const uint64_t* m, int rows, int cols) {
+  int full = 1;
+  for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+    const uint64_t lo = rows >= 64 ? ~0ull : (1ull << rows) - 1;
+    const uint64_t hi = rows <= 64 ? 0ull : rows >= 128 ? ~0ull : (1ull << (rows - 64)) - 1;
+    full &= m[2 * c] == lo && m[2 * c + 1] == hi;
+  }
+  return __syncthreads_and(full);
+}
+
+// Both words of a column filled along it from the set bits of r through the bits of on.
+__device__ __forceinline__ void fill_column(uint64_t (&r)[2], const uint64_t (&on)[2]) {
+#pragma unroll
+  for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      uint64_t u = r[k], p = on[k], d = u, q = p;
+#pragma unroll
+      for (int s = 1; s < 64; s <<= 1) {
+        u |= p & (u << s);
+        p &= p << s;
+        d |= q & (d >> s);
+        q &= q >> s;
+      }
+      r[k] = u | d;
+    }
+    if (pass == 0) {  // across the word boundary, then once more within the words
+      const uint64_t up = (r[0] >> 63) & on[1], dn = (r[1] << 63) & on[0];
+      if (!((up & ~r[1]) | (dn & ~r[0]))) return;
+      r[1] |= up;
+      r[0] |= dn;
+    }
+  }
+}
+
+// bwselect: the connected component of the set bits of on (rows x cols, rows <= 128, cols <= 128)
+// that contains the 0-based seed (sr, sc), 4- or 8-connected, into lab.  All threads of the
+// block call it; a barrier before (on written) is the caller's, the one after is here.
+__device__ inline void flood_bits(const uint64_t* on, uint64_t* lab, int rows, int cols, int sr, int sc, int conn) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const bool seed_ok = sr >= 0 && sr < rows && sc >= 0 && sc < cols && bit_at(on, sr, sc);
+    const int groups = (cols + 31) / 32;  // columns 32 j + lane
+    for (int c = lane; c < cols; c += 32) {
+      lab[2 * c] = seed_ok && c == sc && sr < 64 ? 1ull << sr : 0ull;
+      lab[2 * c + 1] = seed_ok && c == sc && sr >= 64 ? 1ull << (sr - 64) : 0ull;
+    }
+    __syncwarp();
+    // every productive round sets at least one bit, so rows cols rounds bound the loop
+    for (int round = 0; seed_ok && round < rows * cols; ++round) {
+      uint64_t changed = 0;
+      for (int j = 0; j < groups; ++j) {
+        const int c = 32 * j + lane;
+        const bool in = c < cols;
+        uint64_t o[2] = {in ? on[2 * c] : 0ull, in ? on[2 * c + 1] : 0ull};
+        uint64_t r[2] = {in ? lab[2 * c] : 0ull, in ? lab[2 * c + 1] : 0ull};
+        const uint64_t r0 = r[0], r1 = r[1];
+        // from the neighbouring columns (8-connected: their rows one up and down as well)
+#pragma unroll
+        for (int k = -1; k <= 1; k += 2) {
+          const int cn = c + k;
+          if (in && cn >= 0 && cn < cols) {
+            uint64_t a0 = lab[2 * cn], a1 = lab[2 * cn + 1];
+            if (conn == 8) {
+              const uint64_t b0 = a0 | a0 << 1 | a0 >> 1 | a1 << 63, b1 = a1 | a1 << 1 | a1 >> 1 | a0 >> 63;
+              a0 = b0;
+              a1 = b1;
+            }
+            r[0] |= a0 & o[0];
+            r[1] |= a1 & o[1];
+          }
+        }
+        fill_column(r, o);
+        // along the rows through the 32 columns of the group
+        uint64_t p[2] = {o[0], o[1]}, q[2] = {o[0], o[1]}, d[2] = {r[0], r[1]};
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            if (k == 1 && rows <= 64) continue;
+            const uint64_t ru = __shfl_up_sync(0xffffffffu, r[k], s), pu = __shfl_up_sync(0xffffffffu, p[k], s);
+            const uint64_t rd = __shfl_down_sync(0xffffffffu, d[k], s), pd = __shfl_down_sync(0xffffffffu, q[k], s);
+            r[k] |= lane >= s ? p[k] & ru : 0ull;
+            p[k] &= lane >= s ? pu : 0ull;
+            d[k] |= lane + s < 32 ? q[k] & rd : 0ull;
+            q[k] &= lane + s < 32 ? pd : 0ull;
+          }
+        r[0] |= d[0];
+        r[1] |= d[1];
+        changed |= (r[0] ^ r0) | (r[1] ^ r1);
+        __syncwarp();
+        if (in) {
+          lab[2 * c] = r[0];
+          lab[2 * c + 1] = r[1];
+        }
+        __syncwarp();
+      }
+      if (!__any_sync(0xffffffffu, changed != 0)) break;
+    }
+  }
+  __syncthreads();
 }
 
 // MATLAB round(): half away from zero.

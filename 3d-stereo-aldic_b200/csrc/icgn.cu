@@ -30,7 +30,8 @@
 
 namespace aldic {
 
-constexpr int kNT = 128;  // threads per solve CTA
+constexpr int kNT = 128;    // threads per FP32 solve CTA
+constexpr int kNT64 = 512;  // threads per FP64 re-solve CTA
 constexpr int kSlowSubset = 2;   // queue-1 flag of a subset continued by the multi-warp pass
 constexpr int kMovedSubset = 4;  // queue-1 flag of a subset moved to the FP64 re-solve queue
 constexpr int kToFp64 = 5;       // hand-off code of the warp passes: re-solve in FP64
@@ -105,45 +106,52 @@ __device__ __forceinline__ float warp_g(const FrameDev& fr, const SolveCtl& c, f
   return stencil16(fr.def, fr.M, c.base_r + (int)ix, c.base_c + (int)iy, lx - ix, ly - iy);
 }
 
-// Gauss-Jordan inverse of a 6x6 (column-major) with partial pivoting, FP64.
-__device__ void invert6(const double* Hin, double* Hinv) {
-  double A[36], I[36];
-  for (int k = 0; k < 36; ++k) {
-    A[k] = Hin[k];
-    I[k] = (k % 7 == 0) ? 1.0 : 0.0;
+// The inverse of a subset's 6 x 6 Hessian (h: packed upper triangle by rows) into inv (6 x 6
+// row-major) by Gauss-Jordan on [H | I] with partial pivoting, one warp, FP64; aug is 72 doubles of
+// scratch, fac 6.
+__device__ __forceinline__ void invert6_warp(const double* h, double* aug, double* fac, double* inv, int lane) {
+  for (int e = lane; e < 72; e += 32) {
+    const int i = e / 12, j = e % 12;
+    double val = (j - 6 == i) ? 1.0 : 0.0;
+    if (j < 6) {
+      const int r = i < j ? i : j, cc = i < j ? j : i;  // packed upper-triangle index of (r, cc)
+      val = h[r * 6 - r * (r - 1) / 2 + (cc - r)];
+    }
+    aug[e] = val;
   }
+  __syncwarp();
   for (int k = 0; k < 6; ++k) {
-    int piv = k;
-    double best = fabs(A[k + 6 * k]);
-    for (int i = k + 1; i < 6; ++i)
-      if (fabs(A[i + 6 * k]) > best) {
-        best = fabs(A[i + 6 * k]);
-        piv = i;
-      }
-    if (piv != k)
-      for (int j = 0; j < 6; ++j) {
-        double t = A[k + 6 * j];
-        A[k + 6 * j] = A[piv + 6 * j];
-        A[piv + 6 * j] = t;
-        t = I[k + 6 * j];
-        I[k + 6 * j] = I[piv + 6 * j];
-        I[piv + 6 * j] = t;
-      }
-    const double d = A[k + 6 * k];
-    for (int j = 0; j < 6; ++j) {
-      A[k + 6 * j] /= d;
-      I[k + 6 * j] /= d;
-    }
-    for (int i = 0; i < 6; ++i) {
-      if (i == k) continue;
-      const double l = A[i + 6 * k];
-      for (int j = 0; j < 6; ++j) {
-        A[i + 6 * j] -= l * A[k + 6 * j];
-        I[i + 6 * j] -= l * I[k + 6 * j];
+    // the row (>= k) with the largest |entry| in column k, first one on ties
+    double best = lane >= k && lane < 6 ? fabs(aug[lane * 12 + k]) : -1.0;
+    int piv = lane;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      const double ob = __shfl_down_sync(0xffffffffu, best, o);
+      const int op = __shfl_down_sync(0xffffffffu, piv, o);
+      if (lane + o < 8 && (ob > best || (ob == best && op < piv))) {
+        best = ob;
+        piv = op;
       }
     }
+    piv = __shfl_sync(0xffffffffu, piv, 0);
+    if (piv != k && lane < 12) {
+      const double tk = aug[k * 12 + lane];
+      aug[k * 12 + lane] = aug[piv * 12 + lane];
+      aug[piv * 12 + lane] = tk;
+    }
+    __syncwarp();
+    if (lane < 6) fac[lane] = aug[lane * 12 + k];
+    const double pv = aug[k * 12 + k];
+    __syncwarp();
+    if (lane < 12) aug[k * 12 + lane] /= pv;
+    __syncwarp();
+    for (int e = lane; e < 72; e += 32) {
+      const int i = e / 12, j = e % 12;
+      if (i != k) aug[e] -= fac[i] * aug[k * 12 + j];
+    }
+    __syncwarp();
   }
-  for (int k = 0; k < 36; ++k) Hinv[k] = I[k];
+  for (int e = lane; e < 36; e += 32) inv[e] = aug[e / 6 * 12 + 6 + e % 6];
 }
 
 // ================================================================================
@@ -243,7 +251,7 @@ __global__ void icgn_classify_kernel(IcgnArgs a) {
 // 6-DOF solve kernel (general: masks, enlarged windows; FP32, or FP64 for re-solves)
 // ================================================================================
 // Shared-memory arrays of one subset: g (the interpolated deformed window, FP32 or FP64),
-// f, f_x, f_y (FP32 image data), and the u8 masks of the flood fills.
+// f, f_x, f_y (FP32 image data), and the masks of the flood fills as bit columns (PixelBits).
 template <bool F64>
 struct SolveSmem {
   using G = typename std::conditional<F64, double, float>::type;
@@ -251,25 +259,24 @@ struct SolveSmem {
   float* f;
   float* gx;
   float* gy;
-  uint8_t* on;    // f-mask pixel on (quadtree)
-  uint8_t* lab;   // flood-fill output (bw4, then per-iteration g region)
-  uint8_t* tmp;   // flood-fill input
-  uint8_t* fbw8;  // 8-connected f-mask region (g-mask fallback)
+  uint64_t* on;    // f-mask pixel on (quadtree)
+  uint64_t* lab;   // flood-fill output (bw4, then per-iteration g region)
+  uint64_t* tmp;   // flood-fill input
+  uint64_t* fbw8;  // 8-connected f-mask region (g-mask fallback)
 };
 
 template <bool F64>
-__device__ __forceinline__ SolveSmem<F64> carve(unsigned char* base, int npx) {
+__device__ __forceinline__ SolveSmem<F64> carve(unsigned char* base, int npx, int W1) {
   using G = typename SolveSmem<F64>::G;
   SolveSmem<F64> s;
-  s.g = reinterpret_cast<G*>(base);  // first: 8-byte aligned for the FP64 form
+  s.on = reinterpret_cast<uint64_t*>(base);  // first: 8-byte aligned, as the FP64 g after it
+  s.lab = s.on + 2 * W1;
+  s.tmp = s.lab + 2 * W1;
+  s.fbw8 = s.tmp + 2 * W1;
+  s.g = reinterpret_cast<G*>(s.fbw8 + 2 * W1);
   s.f = reinterpret_cast<float*>(s.g + npx);
   s.gx = s.f + npx;
   s.gy = s.gx + npx;
-  uint8_t* u = reinterpret_cast<uint8_t*>(s.gy + npx);
-  s.on = u;
-  s.lab = u + npx;
-  s.tmp = u + 2 * npx;
-  s.fbw8 = u + 3 * npx;
   return s;
 }
 
@@ -306,13 +313,20 @@ __device__ __forceinline__ double fp32_noise(double factor, int step, double bf,
 // passes) and moves subsets whose convergence test is too close to call to queue 2; the FP64
 // form (interpolation in the reference's own double arithmetic, FP64 sums) re-solves queue 2
 // from the initial guesses, so its decisions are the FP64 reference's.
+//
+// Both are bound by the latency of one subset (few subsets, a serial control thread), so the FP64
+// form, whose sums may be split any way, takes 512 threads a subset, and the FP32 form, whose
+// per-thread sums fix 128 threads, runs as many CTAs as fit.  The flood fills work on bit columns
+// (flood_bits), and the g-region fill of an iteration is skipped where no g is zero: its
+// result is the whole window then.  A plate with a hole (2048^2, winsize 32, 17 757 nodes):
+// FP32 kernel 3.22 -> 0.21 ms, FP64 kernel 1.12 -> 0.11 ms a call.
 template <bool F64, int NT>
 __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) {
   using G = typename SolveSmem<F64>::G;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ SolveCtl c;
-  __shared__ double red[(NT / 32) * 40];
-  __shared__ double sums[40];
+  __shared__ double red[(NT / 32) * 37];
+  __shared__ double sums[40], aug[72], fac[6];
   const int tid = threadIdx.x;
   const FrameDev& fr = a.fr;
   const bool quad = (a.variant == 1);
@@ -334,36 +348,50 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
       y0 = mround(y0);
     }
     const int seed = (int)floor((w + 1) / 2.0) - 1;
-    SolveSmem<F64> s = carve<F64>(smem_raw, npx);
+    SolveSmem<F64> s = carve<F64>(smem_raw, npx, W1);
+    const int q_nt = NT / W1, r_nt = NT % W1, aa0 = tid % W1, bb0 = tid / W1;
     // ---- load the subset window ----
     {
       const int r0 = (int)x0 - half - 1, c0 = (int)y0 - half - 1;
+      int aa = aa0, bb = bb0;
       for (int p = tid; p < npx; p += NT) {
-        const int aa = p % W1, bb = p / W1;
         const size_t k = (size_t)(r0 + aa) + (size_t)(c0 + bb) * fr.M;
         const size_t kg = (size_t)(r0 + aa - a.crop) + (size_t)(c0 + bb - a.crop) * gM;
         float f = fr.ref[k];
-        uint8_t on = 1;
-        if (quad && fr.mask) {
-          on = fr.mask[k] != 0;
-          if (!on) f = 0.f;
-        }
+        if (quad && fr.mask && fr.mask[k] == 0) f = 0.f;
         s.f[p] = f;
         s.gx[p] = fr.gx[kg];
         s.gy[p] = fr.gy[kg];
-        s.on[p] = on;
+        aa += r_nt;
+        bb += q_nt;
+        if (aa >= W1) {
+          aa -= W1;
+          bb += 1;
+        }
       }
+      if (quad)
+        build_bits(s.on, W1, W1, NT, [&](int r, int cc) {
+          return !fr.mask || fr.mask[(size_t)(r0 + r) + (size_t)(c0 + cc) * fr.M] != 0;
+        });
     }
     __syncthreads();
     if (masked) {
       // bwselect(logical(mask), seed, seed, 4) restricts f, fx, fy (funICGNQuadtree.m:83-88)
-      flood_select(s.on, s.lab, W1, W1, seed, seed, 4, nullptr);
-      for (int p = tid; p < npx; p += NT)
-        if (!s.lab[p]) {
+      flood_bits(s.on, s.lab, W1, W1, seed, seed, 4);
+      int aa = aa0, bb = bb0;
+      for (int p = tid; p < npx; p += NT) {
+        if (!bit_at(s.lab, aa, bb)) {
           s.f[p] = 0.f;
           s.gx[p] = 0.f;
           s.gy[p] = 0.f;
         }
+        aa += r_nt;
+        bb += q_nt;
+        if (aa >= W1) {
+          aa -= W1;
+          bb += 1;
+        }
+      }
       __syncthreads();
     }
     // ---- setup sums: H (21), sum J f (6), sum J (6), f stats (3), sum |f| (1); FP64 per thread
@@ -372,8 +400,15 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
       double v[37];
 #pragma unroll
       for (int k = 0; k < 37; ++k) v[k] = 0.0;
+      int aa = aa0, bb = bb0;
       for (int p = tid; p < npx; p += NT) {
-        const double dx = (double)(p % W1 - half), dy = (double)(p / W1 - half);
+        const double dx = (double)(aa - half), dy = (double)(bb - half);
+        aa += r_nt;
+        bb += q_nt;
+        if (aa >= W1) {
+          aa -= W1;
+          bb += 1;
+        }
         const double gxv = s.gx[p], gyv = s.gy[p], f = s.f[p];
         const double J[6] = {gxv * dx, gyv * dx, gxv * dy, gyv * dy, gxv, gyv};
 #pragma unroll
@@ -398,20 +433,9 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
       }
       block_sum<37, NT>(v, red, sums);
     }
+    if (tid < 32) invert6_warp(sums, aug, fac, c.Hinv, tid);  // the symmetric 6 x 6 inverse
     if (tid == 0) {
-      double H[36];
-      int k = 0;
-      for (int i = 0; i < 6; ++i)
-        for (int j = i; j < 6; ++j) {
-          H[i + 6 * j] = sums[k];
-          H[j + 6 * i] = sums[k];
-          ++k;
-        }
-      // packed lower triangle by columns == upper triangle by rows
-      k = 0;
-      for (int col = 0; col < 6; ++col)
-        for (int row = col; row < 6; ++row) c.H[k++] = H[row + 6 * col];
-      invert6(H, c.Hinv);
+      for (int k = 0; k < 21; ++k) c.H[k] = sums[k];  // packed lower triangle by columns
       const double n = sums[35];
       if (n > 0) {
         c.meanf = sums[33] / n;
@@ -448,7 +472,6 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
     }
     __syncthreads();
     // ---- Gauss-Newton iterations ----
-    const int q_nt = NT / W1, r_nt = NT % W1;
     while (true) {
       if (tid == 0) {
         int go = (!c.to_fp64 && c.step <= a.max_iter && c.normNew > a.tol && c.normAbs > a.tol) ? 1 : 0;
@@ -483,12 +506,13 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
       }
       __syncthreads();
       if (!c.go) break;
-      // pass 1: interpolate, single-pass sums (FP64 across the threads' partials)
-      double v[11];
+      // pass 1: interpolate and, for a subset without a mask region, the sums (FP64 across the
+      // threads' partials); a masked subset's sums are taken over its g region below
+      int zero = 0;
       {
         G C[6] = {0, 0, 0, 0, 0, 0}, S1 = 0, S2 = 0, fg = 0;
-        float ns = 0.f, nz = 0.f;
-        int aa = tid % W1, bb = tid / W1;
+        float ns = 0.f;
+        int aa = aa0, bb = bb0;
         for (int p = tid; p < npx; p += NT) {
           G g;
           if constexpr (F64) {
@@ -501,23 +525,25 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
           } else {
             g = warp_g(fr, c, (float)(aa - half), (float)(bb - half));
           }
-          s.g[p] = g;
-          const G dx = (G)(aa - half), dy = (G)(bb - half);
-          const G ag = (G)s.gx[p] * g, bg = (G)s.gy[p] * g;
-          C[0] = fma(ag, dx, C[0]);
-          C[1] = fma(bg, dx, C[1]);
-          C[2] = fma(ag, dy, C[2]);
-          C[3] = fma(bg, dy, C[3]);
-          C[4] += ag;
-          C[5] += bg;
-          const bool sel = quad ? (fabs(g) > (G)1e-10) : true;
-          if (sel) {
-            S1 += g;
-            S2 = fma(g, g, S2);
-            ns += 1.f;
+          zero |= g == (G)0;
+          if (quad) s.g[p] = g;
+          if (!masked) {
+            const G dx = (G)(aa - half), dy = (G)(bb - half);
+            const G ag = (G)s.gx[p] * g, bg = (G)s.gy[p] * g;
+            C[0] = fma(ag, dx, C[0]);
+            C[1] = fma(bg, dx, C[1]);
+            C[2] = fma(ag, dy, C[2]);
+            C[3] = fma(bg, dy, C[3]);
+            C[4] += ag;
+            C[5] += bg;
+            const bool sel = quad ? (fabs(g) > (G)1e-10) : true;
+            if (sel) {
+              S1 += g;
+              S2 = fma(g, g, S2);
+              ns += 1.f;
+            }
+            if (want_fg) fg = fma((G)s.f[p], g, fg);
           }
-          nz += (g == (G)0) ? 1.f : 0.f;
-          if (want_fg) fg = fma((G)s.f[p], g, fg);
           aa += r_nt;
           bb += q_nt;
           if (aa >= W1) {
@@ -525,39 +551,44 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
             bb += 1;
           }
         }
+        if (!masked) {
+          double v[10];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = C[k];
-        v[6] = S1;
-        v[7] = S2;
-        v[8] = ns;
-        v[9] = nz;
-        v[10] = fg;
+          for (int k = 0; k < 6; ++k) v[k] = C[k];
+          v[6] = S1;
+          v[7] = S2;
+          v[8] = ns;
+          v[9] = fg;
+          block_sum<10, NT>(v, red, sums);
+        }
       }
-      block_sum<11, NT>(v, red, sums);
-      const bool run_mask = quad && (masked || sums[9] > 0);
-      if (run_mask) {
+      const bool any_zero = __syncthreads_or(zero);
+      if (quad && (masked || any_zero)) {
         // g region: bwselect(logical(g), seed, seed, 8); if it covers the window, the
-        // 8-connected f-mask region instead (funICGNQuadtree.m:170-182)
-        for (int p = tid; p < npx; p += NT) s.tmp[p] = (s.g[p] != (G)0);
-        __syncthreads();
-        flood_select(s.tmp, s.lab, W1, W1, seed, seed, 8, nullptr);
-        int allon = 1;
-        for (int p = tid; p < npx; p += NT) allon &= s.lab[p];
-        allon = __syncthreads_and(allon);
-        const uint8_t* gm = s.lab;
+        // 8-connected f-mask region instead (funICGNQuadtree.m:170-182).  Without a zero in g it
+        // is the window.
+        bool allon = true;
+        if (any_zero) {
+          build_bits(s.tmp, W1, W1, NT, [&](int r, int cc) { return s.g[r + cc * W1] != (G)0; });
+          __syncthreads();
+          flood_bits(s.tmp, s.lab, W1, W1, seed, seed, 8);
+          allon = bits_full(s.lab, W1, W1);
+        }
+        const uint64_t* gm = s.lab;
         if (allon) {
           if (!c.fbw8_ready) {
-            flood_select(s.on, s.fbw8, W1, W1, seed, seed, 8, nullptr);
+            flood_bits(s.on, s.fbw8, W1, W1, seed, seed, 8);
             if (tid == 0) c.fbw8_ready = 1;
           }
           gm = s.fbw8;
         }
-        __syncthreads();
         G C2[6] = {0, 0, 0, 0, 0, 0}, T1 = 0, T2 = 0, TF = 0;
         float tn = 0.f, gs = 0.f;
+        int aa = aa0, bb = bb0;
         for (int p = tid; p < npx; p += NT) {
-          const G dx = (G)(p % W1 - half), dy = (G)(p / W1 - half);
-          const G g = gm[p] ? s.g[p] : (G)0;
+          const G dx = (G)(aa - half), dy = (G)(bb - half);
+          const bool on = bit_at(gm, aa, bb);
+          const G g = on ? s.g[p] : (G)0;
           const G ag = (G)s.gx[p] * g, bg = (G)s.gy[p] * g;
           C2[0] = fma(ag, dx, C2[0]);
           C2[1] = fma(bg, dx, C2[1]);
@@ -570,12 +601,18 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
             T2 = fma(g, g, T2);
             tn += 1.f;
           }
-          gs += gm[p] ? 1.f : 0.f;
+          gs += on ? 1.f : 0.f;
           if (want_fg) TF = fma((G)s.f[p], g, TF);
+          aa += r_nt;
+          bb += q_nt;
+          if (aa >= W1) {
+            aa -= W1;
+            bb += 1;
+          }
         }
-        double v2[11] = {C2[0], C2[1], C2[2], C2[3], C2[4], C2[5], T1, T2, tn, gs, TF};
+        double v2[11] = {C2[0], C2[1], C2[2], C2[3], C2[4], C2[5], T1, T2, tn, TF, gs};
         block_sum<11, NT>(v2, red, sums);
-        if (tid == 0) c.gsum_prev = sums[9];
+        if (tid == 0) c.gsum_prev = sums[10];
       }
       if (tid == 0) {
         const double n = sums[8];
@@ -589,7 +626,7 @@ __global__ void __launch_bounds__(NT) icgn_solve_kernel(IcgnArgs a, int bucket) 
         }
         double b[6];
         for (int i = 0; i < 6; ++i) b[i] = c.bf * (c.A[i] - (sums[i] - meang * c.B[i]) / bg);
-        if (want_fg) c.znssd = 2.0 - 2.0 * (sums[10] - c.meanf * sums[6]) / (c.bf * bg);
+        if (want_fg) c.znssd = 2.0 - 2.0 * (sums[9] - c.meanf * sums[6]) / (c.bf * bg);
         double nn = 0;
         for (int i = 0; i < 6; ++i) nn += b[i] * b[i];
         c.normNew = sqrt(nn);
@@ -806,26 +843,25 @@ struct Sub1Ctl {
   int step, go, status, fbw8_ready;
 };
 
-// Shared-memory arrays of one Subpb1 subset: f (= ImgRef .* mask), fx, fy, g as floats;
-// on (mask pixel set), cur (the region that currently restricts f, fx, fy: bw4 after
-// set-up, the last g region after a masked iteration), tmp/glab (flood fill of g), fbw8.
+// Shared-memory arrays of one Subpb1 subset: f (= ImgRef .* mask), fx, fy, g as floats; as bit
+// columns on (mask pixel set), cur (the region that currently restricts f, fx, fy: bw4 after
+// set-up, the last g region after a masked iteration), tmp / glab (flood fill of g), fbw8.
 struct Sub1Smem {
   float *f, *gx, *gy, *g;
-  uint8_t *on, *cur, *tmp, *glab, *fbw8;
+  uint64_t *on, *cur, *tmp, *glab, *fbw8;
 };
 
-__device__ __forceinline__ Sub1Smem carve_sub1(unsigned char* base, int npx) {
+__device__ __forceinline__ Sub1Smem carve_sub1(unsigned char* base, int npx, int cols) {
   Sub1Smem s;
-  s.f = reinterpret_cast<float*>(base);
+  s.on = reinterpret_cast<uint64_t*>(base);
+  s.cur = s.on + 2 * cols;
+  s.tmp = s.cur + 2 * cols;
+  s.glab = s.tmp + 2 * cols;
+  s.fbw8 = s.glab + 2 * cols;
+  s.f = reinterpret_cast<float*>(s.fbw8 + 2 * cols);
   s.gx = s.f + npx;
   s.gy = s.gx + npx;
   s.g = s.gy + npx;
-  uint8_t* u = reinterpret_cast<uint8_t*>(s.g + npx);
-  s.on = u;
-  s.cur = u + npx;
-  s.tmp = u + 2 * npx;
-  s.glab = u + 3 * npx;
-  s.fbw8 = u + 4 * npx;
   return s;
 }
 
@@ -882,36 +918,45 @@ __global__ void __launch_bounds__(kNT) subpb1_solve_kernel(Sub1Args a, int bucke
     // (funICGN_Subpb1quadtree.m:93)
     const int sc = (int)floor((wx + 1) / 2.0) - 1;
     const int sr = (int)floor((wy + 1) / 2.0) - 1;
-    Sub1Smem s = carve_sub1(smem_raw, npx);
+    Sub1Smem s = carve_sub1(smem_raw, npx, Cc);
+    const int q_nt = kNT / R, r_nt = kNT % R, aa0 = tid % R, bb0 = tid / R;
     {
       const int r0 = (int)x0 - hx - 1, c0 = (int)y0 - hy - 1;
+      int aa = aa0, bb = bb0;
       for (int p = tid; p < npx; p += kNT) {
-        const int aa = p % R, bb = p / R;
         const size_t k = (size_t)(r0 + aa) + (size_t)(c0 + bb) * fr.M;
         const size_t kg = (size_t)(r0 + aa - 3) + (size_t)(c0 + bb - 3) * gM;
         float f = fr.ref[k];
-        uint8_t on = 1;
-        if (quad && fr.mask) {
-          on = fr.mask[k] != 0;
-          if (!on) f = 0.f;
-        }
+        if (quad && fr.mask && fr.mask[k] == 0) f = 0.f;
         s.f[p] = f;
         s.gx[p] = fr.gx[kg];
         s.gy[p] = fr.gy[kg];
-        s.on[p] = on;
-        s.cur[p] = 1;
+        aa += r_nt;
+        bb += q_nt;
+        if (aa >= R) {
+          aa -= R;
+          bb += 1;
+        }
       }
+      build_bits(s.on, R, Cc, kNT, [&](int r, int cc) {
+        return !quad || !fr.mask || fr.mask[(size_t)(r0 + r) + (size_t)(c0 + cc) * fr.M] != 0;
+      });
+      if (!masked) build_bits(s.cur, R, Cc, kNT, [](int, int) { return true; });
     }
     __syncthreads();
-    if (masked) {
-      flood_select(s.on, s.cur, R, Cc, sr, sc, 4, nullptr);  // cur = bw4
-      __syncthreads();
-    }
+    if (masked) flood_bits(s.on, s.cur, R, Cc, sr, sc, 4);  // cur = bw4
     // f-side sums restricted by cur: H(3), sum J f (2), sum J (2), f stats (3), sum|f|
     {
       float h0 = 0, h1 = 0, h2 = 0, jf0 = 0, jf1 = 0, jb0 = 0, jb1 = 0, fs = 0, fs2 = 0, fn = 0, fab = 0;
+      int aa = aa0, bb = bb0;
       for (int p = tid; p < npx; p += kNT) {
-        const float m = s.cur[p] ? 1.f : 0.f;
+        const float m = bit_at(s.cur, aa, bb) ? 1.f : 0.f;
+        aa += r_nt;
+        bb += q_nt;
+        if (aa >= R) {
+          aa -= R;
+          bb += 1;
+        }
         const float gxv = s.gx[p] * m, gyv = s.gy[p] * m, f = s.f[p] * m;
         h0 = fmaf(gxv, gxv, h0);
         h1 = fmaf(gxv, gyv, h1);
@@ -979,52 +1024,78 @@ __global__ void __launch_bounds__(kNT) subpb1_solve_kernel(Sub1Args a, int bucke
       }
       __syncthreads();
       if (!c.go) break;
-      // pass 1: g and the g-side sums with the current f-side region
-      float C0 = 0, C1 = 0, S1 = 0, S2 = 0, ns = 0, nz = 0;
-      for (int p = tid; p < npx; p += kNT) {
-        const float dx = (float)(p % R - hx), dy = (float)(p / R - hy);
-        const float lx = dx + fmaf(c.pf[0], dx, fmaf(c.pf[2], dy, c.f5));
-        const float ly = dy + fmaf(c.pf[3], dy, fmaf(c.pf[1], dx, c.f6));
-        const float ix = floorf(lx), iy = floorf(ly);
-        const float g = stencil16(fr.def, fr.M, c.base_r + (int)ix, c.base_c + (int)iy, lx - ix, ly - iy);
-        s.g[p] = g;
-        const float m = s.cur[p] ? 1.f : 0.f;
-        C0 = fmaf(s.gx[p] * m, g, C0);
-        C1 = fmaf(s.gy[p] * m, g, C1);
-        const bool sel = quad ? (fabsf(g) > 1e-10f) : true;
-        if (sel) {
-          S1 += g;
-          S2 = fmaf(g, g, S2);
-          ns += 1.f;
+      // pass 1: g and, for a subset without a mask region, the g-side sums with the current
+      // f-side region; a masked subset's sums are taken over its g region below
+      float C0 = 0, C1 = 0, S1 = 0, S2 = 0, ns = 0;
+      int zero = 0;
+      {
+        int aa = aa0, bb = bb0;
+        for (int p = tid; p < npx; p += kNT) {
+          const float dx = (float)(aa - hx), dy = (float)(bb - hy);
+          const float lx = dx + fmaf(c.pf[0], dx, fmaf(c.pf[2], dy, c.f5));
+          const float ly = dy + fmaf(c.pf[3], dy, fmaf(c.pf[1], dx, c.f6));
+          const float ix = floorf(lx), iy = floorf(ly);
+          const float g = stencil16(fr.def, fr.M, c.base_r + (int)ix, c.base_c + (int)iy, lx - ix, ly - iy);
+          s.g[p] = g;
+          zero |= g == 0.f;
+          if (!masked) {
+            const float m = bit_at(s.cur, aa, bb) ? 1.f : 0.f;
+            C0 = fmaf(s.gx[p] * m, g, C0);
+            C1 = fmaf(s.gy[p] * m, g, C1);
+            const bool sel = quad ? (fabsf(g) > 1e-10f) : true;
+            if (sel) {
+              S1 += g;
+              S2 = fmaf(g, g, S2);
+              ns += 1.f;
+            }
+          }
+          aa += r_nt;
+          bb += q_nt;
+          if (aa >= R) {
+            aa -= R;
+            bb += 1;
+          }
         }
-        nz += (g == 0.f) ? 1.f : 0.f;
       }
-      double gv[6] = {C0, C1, S1, S2, ns, nz};
-      block_sum<6, kNT>(gv, red, sums);
-      double Cg[2] = {sums[0], sums[1]}, Sg1 = sums[2], Sg2 = sums[3], Sgn = sums[4];
-      const bool run_mask = quad && (masked || sums[5] > 0);
-      __syncthreads();
-      if (run_mask) {
+      double Cg[2] = {0, 0}, Sg1 = 0, Sg2 = 0, Sgn = 0;
+      if (!masked) {
+        double gv[5] = {C0, C1, S1, S2, ns};
+        block_sum<5, kNT>(gv, red, sums);
+        Cg[0] = sums[0];
+        Cg[1] = sums[1];
+        Sg1 = sums[2];
+        Sg2 = sums[3];
+        Sgn = sums[4];
+      }
+      const bool any_zero = __syncthreads_or(zero);
+      if (quad && (masked || any_zero)) {
         // funICGN_Subpb1quadtree.m:158-193: 4-connected g region, fallback to the
-        // 8-connected f-mask region; f, fx, fy, H, mean_f, bf recomputed on it.
-        for (int p = tid; p < npx; p += kNT) s.tmp[p] = (s.g[p] != 0.f);
-        __syncthreads();
-        flood_select(s.tmp, s.glab, R, Cc, sr, sc, 4, nullptr);
-        int allon = 1;
-        for (int p = tid; p < npx; p += kNT) allon &= s.glab[p];
-        allon = __syncthreads_and(allon);
-        if (allon && !c.fbw8_ready) {
-          flood_select(s.on, s.fbw8, R, Cc, sr, sc, 8, nullptr);
+        // 8-connected f-mask region; f, fx, fy, H, mean_f, bf recomputed on it.  Without a zero
+        // in g the g region is the window.
+        bool allon = true;
+        if (any_zero) {
+          build_bits(s.tmp, R, Cc, kNT, [&](int r, int cc) { return s.g[r + cc * R] != 0.f; });
           __syncthreads();
+          flood_bits(s.tmp, s.glab, R, Cc, sr, sc, 4);
+          allon = bits_full(s.glab, R, Cc);
+        }
+        if (allon && !c.fbw8_ready) {
+          flood_bits(s.on, s.fbw8, R, Cc, sr, sc, 8);
           if (tid == 0) c.fbw8_ready = 1;
         }
-        const uint8_t* gm = allon ? s.fbw8 : s.glab;
+        const uint64_t* gm = allon ? s.fbw8 : s.glab;
+        for (int k = tid; k < 2 * Cc; k += kNT) s.cur[k] = gm[k];
         float h0 = 0, h1 = 0, h2 = 0, jf0 = 0, jf1 = 0, jb0 = 0, jb1 = 0, fs = 0, fs2 = 0, fn = 0, fab = 0;
         float c0 = 0, c1 = 0, t1 = 0, t2 = 0, tn = 0;
+        int aa = aa0, bb = bb0;
         for (int p = tid; p < npx; p += kNT) {
-          const uint8_t mk = gm[p];
-          s.cur[p] = mk;
-          const float m = mk ? 1.f : 0.f;
+          const float m = bit_at(gm, aa, bb) ? 1.f : 0.f;
+          aa += r_nt;
+          bb += q_nt;
+          if (aa >= R) {
+            aa -= R;
+            bb += 1;
+          }
           const float gxv = s.gx[p] * m, gyv = s.gy[p] * m, f = s.f[p] * m, g = s.g[p] * m;
           h0 = fmaf(gxv, gxv, h0);
           h1 = fmaf(gxv, gyv, h1);
@@ -1115,8 +1186,15 @@ static int occupancy_grid(const void* fn, size_t smem, int threads = kNT) {
   return sms * per_sm;
 }
 
+// The limits of the entry points (windows above them are refused, or not re-solved in FP64).
 size_t icgn_smem_bytes(int w) { return (size_t)(w + 1) * (w + 1) * (4 * sizeof(float) + 4); }
 size_t icgn_smem_bytes_f64(int w) { return (size_t)(w + 1) * (w + 1) * (sizeof(double) + 3 * sizeof(float) + 4); }
+// What icgn_solve_kernel takes (carve): never more than the limits above.
+template <bool F64>
+static size_t solve_smem_bytes(int w) {
+  const size_t W1 = w + 1;
+  return W1 * W1 * ((F64 ? sizeof(double) : sizeof(float)) + 3 * sizeof(float)) + 8 * W1 * sizeof(uint64_t);
+}
 size_t sub1_smem_bytes(int wx, int wy) { return (size_t)(wx + 1) * (wy + 1) * (4 * sizeof(float) + 5); }
 
 
@@ -1353,28 +1431,20 @@ int launch_icgn(const IcgnArgs& a, int wmax_enlarged, cudaStream_t st) {
     launches += a.slow_nw == 4 ? launch_icgn_tile<4, true>(a, geo, sms, st)
                                : launch_icgn_tile<kSlowNW, true>(a, geo, sms, st);
   {  // enlarged / masked subsets, and those handed over by the fast kernel
-    const size_t smem = icgn_smem_bytes(wmax_enlarged);
+    const size_t smem = solve_smem_bytes<false>(wmax_enlarged);
     cudaFuncSetAttribute(icgn_solve_kernel<false, kNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int grid = occupancy_grid((const void*)icgn_solve_kernel<false, kNT>, smem, kNT);
-    grid = grid < 296 ? grid : 296;
     if ((long long)grid > a.n) grid = (int)a.n;
-    if (grid < 1) grid = 1;
     icgn_solve_kernel<false, kNT><<<grid, kNT, smem, st>>>(a, 1);
     ++launches;
   }
   if ((a.band > 0 || a.slow_fp64) && a.variant != 2) {
     // FP64 re-solves: the subsets too close to call in FP32 and the long trajectories
-    const size_t smem = icgn_smem_bytes_f64(wmax_enlarged);
-    auto kf = a.fp64_threads == 512   ? icgn_solve_kernel<true, 512>
-              : a.fp64_threads == 256 ? icgn_solve_kernel<true, 256>
-                                      : icgn_solve_kernel<true, 128>;
-    const int nt = a.fp64_threads == 512 ? 512 : (a.fp64_threads == 256 ? 256 : 128);
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int grid = occupancy_grid((const void*)kf, smem, nt);
-    grid = grid < 4 * sms ? grid : 4 * sms;
+    const size_t smem = solve_smem_bytes<true>(wmax_enlarged);
+    cudaFuncSetAttribute(icgn_solve_kernel<true, kNT64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int grid = occupancy_grid((const void*)icgn_solve_kernel<true, kNT64>, smem, kNT64);
     if ((long long)grid > a.n) grid = (int)a.n;
-    if (grid < 1) grid = 1;
-    kf<<<grid, nt, smem, st>>>(a, 2);
+    icgn_solve_kernel<true, kNT64><<<grid, kNT64, smem, st>>>(a, 2);
     ++launches;
   }
   return launches;
@@ -1483,12 +1553,11 @@ int launch_subpb1(const Sub1Args& a, int wmax_x, int wmax_y, cudaStream_t st) {
     launches += 2;
   }
   {  // masked subsets and restarts: the general kernel on queue 1
-    const size_t smem = sub1_smem_bytes(wmax_x, wmax_y);
+    // carve_sub1; never more than sub1_smem_bytes, the entry point's limit
+    const size_t smem = (size_t)(wmax_x + 1) * (wmax_y + 1) * 4 * sizeof(float) + 10 * (wmax_y + 1) * sizeof(uint64_t);
     cudaFuncSetAttribute(subpb1_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int grid = occupancy_grid((const void*)subpb1_solve_kernel, smem);
-    grid = grid < 296 ? grid : 296;
     if ((long long)grid > a.n) grid = (int)a.n;
-    if (grid < 1) grid = 1;
     subpb1_solve_kernel<<<grid, kNT, smem, st>>>(a, 1);
     ++launches;
   }

@@ -412,54 +412,6 @@ __device__ __forceinline__ void pixel_sums(const FrameDev& fr, const WarpF& w, u
   out.nz = nz;
 }
 
-// The inverse of a group's 6 x 6 Hessian (h: packed upper triangle by rows) into inv (6 x 6
-// row-major) by Gauss-Jordan on [H | I] with partial pivoting, one warp, FP64; aug is 72 doubles of
-// scratch, fac 6.
-__device__ __forceinline__ void invert6_warp(const double* h, double* aug, double* fac, double* inv, int lane) {
-  for (int e = lane; e < 72; e += 32) {
-    const int i = e / 12, j = e % 12;
-    double val = (j - 6 == i) ? 1.0 : 0.0;
-    if (j < 6) {
-      const int r = i < j ? i : j, cc = i < j ? j : i;  // packed upper-triangle index of (r, cc)
-      val = h[r * 6 - r * (r - 1) / 2 + (cc - r)];
-    }
-    aug[e] = val;
-  }
-  __syncwarp();
-  for (int k = 0; k < 6; ++k) {
-    // the row (>= k) with the largest |entry| in column k, first one on ties
-    double best = lane >= k && lane < 6 ? fabs(aug[lane * 12 + k]) : -1.0;
-    int piv = lane;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-      const double ob = __shfl_down_sync(0xffffffffu, best, o);
-      const int op = __shfl_down_sync(0xffffffffu, piv, o);
-      if (lane + o < 8 && (ob > best || (ob == best && op < piv))) {
-        best = ob;
-        piv = op;
-      }
-    }
-    piv = __shfl_sync(0xffffffffu, piv, 0);
-    if (piv != k && lane < 12) {
-      const double tk = aug[k * 12 + lane];
-      aug[k * 12 + lane] = aug[piv * 12 + lane];
-      aug[piv * 12 + lane] = tk;
-    }
-    __syncwarp();
-    if (lane < 6) fac[lane] = aug[lane * 12 + k];
-    const double pv = aug[k * 12 + k];
-    __syncwarp();
-    if (lane < 12) aug[k * 12 + lane] /= pv;
-    __syncwarp();
-    for (int e = lane; e < 72; e += 32) {
-      const int i = e / 12, j = e % 12;
-      if (i != k) aug[e] -= fac[i] * aug[k * 12 + j];
-    }
-    __syncwarp();
-  }
-  for (int e = lane; e < 36; e += 32) inv[e] = aug[e / 6 * 12 + 6 + e % 6];
-}
-
 template <int NW, bool SLOW, bool QUAD, bool FG>
 __global__ void __launch_bounds__(32 * NW * kTileGroups, 8 / NW) icgn_tile_kernel(IcgnArgs a, TileGeom geo) {
   constexpr int NG = kTileGroups, GT = 32 * NW;
