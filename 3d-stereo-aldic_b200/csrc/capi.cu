@@ -1195,7 +1195,7 @@ int aldic_subpb2(aldic_ctx* c, int64_t n, const double* coords, int64_t n_el, co
     if (rc) return rc;
   }
   // device buffers: inputs staged, the mesh tables (unless resident), K_e / b_e, the CG vectors
-  const size_t nb = (size_t)subpb2_blocks(n);
+  const int blocks = subpb2_cg_blocks(n);
   Arg ac{coords, (size_t)n * 16, false, nullptr}, au{U, (size_t)n * 16, false, nullptr},
       af{F, (size_t)n * 32, false, nullptr}, ao{Uhat, (size_t)n * 16, true, nullptr};
   c->arena.used = 0;
@@ -1205,8 +1205,8 @@ int aldic_subpb2(aldic_ctx* c, int64_t n, const double* coords, int64_t n_el, co
     if (!is_device_ptr(a->user)) need += ((a->bytes + 255) & ~size_t(255)) + 256;
   const size_t two_n = (size_t)n * 16;
   if (!resident) need += sp2_bytes(n, n_el, adj.size()) + 256;
-  need += (size_t)n_el * (64 + 16) * 8 + 6 * two_n + (size_t)n * 8 + nb * 16 + subpb2_scalars_bytes() + 64 +
-          16 * 256;
+  need += (size_t)n_el * (64 + 16) * 8 + 5 * two_n + (size_t)n * 8 + subpb2_ell_bytes(n) +
+          subpb2_parts_bytes(blocks) + subpb2_scalars_bytes() + 64 + 16 * 256;
   int rc = arena_reserve(c, need);
   if (rc) return rc;
   for (Arg* a : {&ac, &au, &af, &ao}) {
@@ -1235,31 +1235,33 @@ int aldic_subpb2(aldic_ctx* c, int64_t n, const double* coords, int64_t n_el, co
   }
   double* Ke = (double*)arena_take(c, (size_t)n_el * 64 * 8);
   double* be = (double*)arena_take(c, (size_t)n_el * 16 * 8);
-  double* b = (double*)arena_take(c, two_n);
   double* r = (double*)arena_take(c, two_n);
   double* z = (double*)arena_take(c, two_n);
-  double* p = (double*)arena_take(c, two_n);
+  double* p0 = (double*)arena_take(c, two_n);
+  double* p1 = (double*)arena_take(c, two_n);
   double* q = (double*)arena_take(c, two_n);
   double* D = (double*)arena_take(c, (size_t)n * 8);
-  double* part = (double*)arena_take(c, nb * 16);
+  void* ell = arena_take(c, subpb2_ell_bytes(n));
+  void* parts = arena_take(c, subpb2_parts_bytes(blocks));
   Subpb2Scalars* sc = (Subpb2Scalars*)arena_take(c, subpb2_scalars_bytes() + 64);
   double* x = (double*)ao.dev;  // the solution builds in the output
   int l = launch_subpb2_setup((int)n_el, dE, (const double*)ac.dev, n, (const double*)au.dev, (const double*)af.dev,
-                              gauss_order, beta, mu, alpha, dptr, dadj, dkind, Ke, be, b, D, x, r, z, p, part, sc,
-                              c->stream);
-  // batches of 16 iterations; the scalars are read back between batches (the kernels of a
-  // batch that starts after convergence return at once)
+                              gauss_order, beta, mu, alpha, dptr, dadj, dkind, Ke, be, ell, D, x, r, c->stream);
+  // the whole solve in one launch; a launch ends after kSp2Iters iterations at the latest (some
+  // tens of milliseconds), and the next continues it
+  constexpr int kSp2Iters = 4096;
   std::vector<unsigned char> host_sc(subpb2_scalars_bytes());
-  int it = 0, done = 0, ok = 0;
-  for (int launched = 0; launched < maxit;) {
-    const int k = std::min(16, maxit - launched);
-    l += launch_subpb2_iterations(k, (int)n_el, dE, n, dptr, dadj, Ke, dkind, D, x, r, z, p, q, part, tol * tol,
-                                  maxit, sc, c->stream);
-    launched += k;
+  int it = 0, done = 0, ok = 0, timeout = 0;
+  for (int launched = 0; launched < maxit && !done; launched += kSp2Iters) {
+    l += launch_subpb2_cg(launched == 0, std::min(kSp2Iters, maxit - launched), blocks, n, dptr, dadj, dE, (int)n_el,
+                          Ke, dkind, ell, D, x, r, z, p0, p1, q, parts, tol * tol, maxit, sc, c->stream);
     CK(cudaMemcpyAsync(host_sc.data(), sc, host_sc.size(), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    subpb2_read_status(host_sc.data(), &it, &done, &ok);
-    if (done) break;
+    subpb2_read_status(host_sc.data(), &it, &done, &ok, &timeout);
+    if (timeout) {
+      c->launches += l;
+      return fail(c, ALDIC_ERR_TIMEOUT, "the global step's grid barrier timed out");
+    }
   }
   if (info) {
     info[0] = it;

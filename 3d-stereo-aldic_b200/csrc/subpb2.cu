@@ -202,214 +202,351 @@ __host__ __device__ inline void subpb2_gather_row(long long i, const int* adj_pt
   }
 }
 
-// CG scalars, one set for the interleaved 2 n system.
+// State of the solve, one set for the interleaved 2 n system.
 struct Subpb2Scalars {
-  double rz, alpha, beta, rr0, rr;
-  int it, done, ok;
+  double rz, rr0, beta;
+  int it, done, ok, timeout;
+  unsigned int arrived;  // grid barrier: CTAs arrived since the launch
 };
 
 namespace {
 
-constexpr int kSubpb2Threads = 256;
+constexpr int kCgThreads = 128;
+constexpr int kEll = 32;          // entries of a matrix row; a node with more neighbours gathers from K_e
+constexpr int kEllOverflow = 255;
+constexpr int kAsmThreads = 64;
+constexpr long long kBarrierSpins = 20000000LL;  // some seconds of polling
 
-__device__ __forceinline__ void block_partial(double v0, double v1, double* part) {
-  __shared__ double red[2][kSubpb2Threads / 32];
-  v0 = warp_sum(v0);
-  v1 = warp_sum(v1);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) {
-    red[0][wid] = v0;
-    red[1][wid] = v1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s0 = 0.0, s1 = 0.0;
-    for (int k = 0; k < kSubpb2Threads / 32; ++k) {
-      s0 += red[0][k];
-      s1 += red[1][k];
+}  // namespace
+
+// Per node: the rows of the assembled matrix (column numbers and values, one row per thread in
+// column-major ELL arrays of n rows, so that consecutive threads read consecutive entries), the
+// right-hand side (into r), the Jacobi diagonal and the start x = U at dirichlet nodes, 0
+// elsewhere.  free_[i]: 1 free, 2 dirichlet, 0 neither (only free rows are kept).
+__global__ void __launch_bounds__(kAsmThreads) subpb2_assemble_kernel(
+    long long n, const int* __restrict__ adj_ptr, const int* __restrict__ adj, const int* __restrict__ elem, int n_el,
+    const double* __restrict__ Ke, const double* __restrict__ be, const unsigned char* __restrict__ free_,
+    const double* __restrict__ U, double* __restrict__ r, double* __restrict__ D, double* __restrict__ x,
+    int* __restrict__ col, double* __restrict__ val, unsigned char* __restrict__ cnt) {
+  __shared__ int sc[kEll][kAsmThreads];
+  __shared__ double sv[kEll][kAsmThreads];
+  const int t = threadIdx.x;
+  const long long i = blockIdx.x * (long long)kAsmThreads + t;
+  if (i >= n) return;
+  const int kind = free_[i];
+  double bx = 0.0, by = 0.0, dg = 0.0;
+  int m = 0;
+  if (kind == 1)
+    for (int q = adj_ptr[i]; q < adj_ptr[i + 1]; ++q) {
+      const int e = adj[q] >> 3, s = adj[q] & 7;
+      const double* kr = Ke + (long long)e * 64 + s * 8;
+      bx += be[(long long)e * 16 + 2 * s];
+      by += be[(long long)e * 16 + 2 * s + 1];
+      dg += kr[s];
+      for (int b = 0; b < 8; ++b) {
+        const int nb = elem[e + (long long)b * n_el] - 1;
+        if (nb < 0 || m == kEllOverflow) continue;
+        int k = 0;
+        while (k < m && sc[k][t] != nb) ++k;
+        if (k < m) {
+          sv[k][t] += kr[b];
+        } else if (m < kEll) {
+          sc[m][t] = nb;
+          sv[m][t] = kr[b];
+          ++m;
+        } else {
+          m = kEllOverflow;
+        }
+      }
     }
-    part[2 * blockIdx.x] = s0;
-    part[2 * blockIdx.x + 1] = s1;
-  }
+  cnt[i] = (unsigned char)m;
+  if (m != kEllOverflow)
+    for (int k = 0; k < m; ++k) {
+      col[k * n + i] = sc[k][t];
+      val[k * n + i] = sv[k][t];
+    }
+  r[2 * i] = bx;
+  r[2 * i + 1] = by;
+  D[i] = dg;
+  x[2 * i] = kind == 2 ? U[2 * i] : 0.0;
+  x[2 * i + 1] = kind == 2 ? U[2 * i + 1] : 0.0;
 }
 
-// Fixed-order sum of the per-block partials (one block).
-__device__ __forceinline__ void sum_partials(const double* part, int nparts, double& s0, double& s1) {
-  __shared__ double red[2][kSubpb2Threads];
-  double a0 = 0.0, a1 = 0.0;
-  for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
-    a0 += part[2 * k];
-    a1 += part[2 * k + 1];
+namespace {
+
+// Grid barrier that exchanges two sums: every CTA stores its partials of v0, v1, arrives at one
+// counter, and after the barrier adds all CTAs' partials in CTA order, so all get the same bits.
+// (Flag slots that carry the values and are polled by every CTA were slower: 3.5 us against
+// 1.2 us for the counter on 139 CTAs.)  Partials alternate between two sets: a CTA is at most one
+// barrier ahead of one that still reads.  False after a time-out of the wait, which ends every CTA
+// at this or its next barrier.  Every thread calls it; writes before it are visible to all CTAs
+// after it (cooperative launch).
+__device__ __forceinline__ bool grid_exchange(double2* parts, unsigned int& epoch, Subpb2Scalars* sc, double& v0,
+                                              double& v1, double* red) {
+  ++epoch;
+  double2* set = parts + (size_t)gridDim.x * (epoch & 1);
+  v0 = warp_sum(v0);
+  v1 = warp_sum(v1);
+  const int wid = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    red[2 * wid] = v0;
+    red[2 * wid + 1] = v1;
   }
-  red[0][threadIdx.x] = a0;
-  red[1][threadIdx.x] = a1;
   __syncthreads();
+  int late = 0;
   if (threadIdx.x == 0) {
-    double t0 = 0.0, t1 = 0.0;
-    for (int k = 0; k < (int)blockDim.x; ++k) {
-      t0 += red[0][k];
-      t1 += red[1][k];
+    double2 v = make_double2(red[0], red[1]);
+#pragma unroll
+    for (int k = 1; k < kCgThreads / 32; ++k) {
+      v.x += red[2 * k];
+      v.y += red[2 * k + 1];
     }
-    s0 = t0;
-    s1 = t1;
+    __stcg(set + blockIdx.x, v);
+    __threadfence();  // this CTA's writes (ordered by the barrier above) before its arrival
+    atomicAdd(&sc->arrived, 1u);
+    const unsigned int target = epoch * gridDim.x;
+    long long spins = 0;
+    unsigned int seen;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&sc->arrived) : "memory");
+    } while (seen < target && ++spins < kBarrierSpins);
+    late = seen < target;
+    if (late) atomicExch(&sc->timeout, 1);
   }
+  late = __syncthreads_or(late);
+  double s0 = 0.0, s1 = 0.0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += kCgThreads) {
+    const double2 v = __ldcg(set + k);
+    s0 += v.x;
+    s1 += v.y;
+  }
+  s0 = warp_sum(s0);
+  s1 = warp_sum(s1);
+  if ((threadIdx.x & 31) == 0) {
+    red[2 * wid] = s0;
+    red[2 * wid + 1] = s1;
+  }
+  __syncthreads();
+  v0 = v1 = 0.0;
+#pragma unroll
+  for (int k = 0; k < kCgThreads / 32; ++k) {
+    v0 += red[2 * k];
+    v1 += red[2 * k + 1];
+  }
+  __syncthreads();  // red is free again
+  return !late;
 }
 
 }  // namespace
 
-// b, the Jacobi diagonal and the start: x = U at dirichlet nodes (0 elsewhere), then (second
-// kernel) r = b - K x, z = r / D, p = z on the free nodes.  free[i]: 1 free, 2 dirichlet, 0
-// neither.
-__global__ void subpb2_rhs_kernel(long long n, const int* __restrict__ adj_ptr, const int* __restrict__ adj,
-                                  const double* __restrict__ Ke, const double* __restrict__ be,
-                                  const unsigned char* __restrict__ free_, const double* __restrict__ U,
-                                  double* __restrict__ b, double* __restrict__ D, double* __restrict__ x) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double bx = 0.0, by = 0.0, dg = 0.0;
-  for (int q = adj_ptr[i]; q < adj_ptr[i + 1]; ++q) {
-    const int e = adj[q] >> 3, s = adj[q] & 7;
-    bx += be[(long long)e * 16 + 2 * s];
-    by += be[(long long)e * 16 + 2 * s + 1];
-    dg += Ke[(long long)e * 64 + s * 9];
-  }
-  b[2 * i] = bx;
-  b[2 * i + 1] = by;
-  D[i] = dg;
-  const bool dir = free_[i] == 2;
-  x[2 * i] = dir ? U[2 * i] : 0.0;
-  x[2 * i + 1] = dir ? U[2 * i + 1] : 0.0;
-}
+// The whole Jacobi-preconditioned conjugate-gradient solve (or its next `iters` iterations) in one
+// cooperative launch.  Per iteration two grid barriers: after q = K p (with the sum p q) and after
+// the update of x, r, z (with the sums r z and r r).  The new direction p = z + beta p_old is
+// formed where it is read, by the node and by its neighbours, and kept in the other of two
+// buffers, which saves a third barrier.  ONE: a thread has one node and keeps its x, r, D and the
+// first kEllRegs entries of its matrix row in registers.
+//
+// What bounds it: the latency of the barriers and gathers (17 757 nodes: the matrix and the
+// vectors are 5 MB in L2).  Five launches an iteration and a host read-back every 16 took 872 us
+// a solve of 30 iterations; one launch with every row read from L2 436 us; this form 275 us (185 us in the kernel).
+constexpr int kEllRegs = 12;
 
-__global__ void subpb2_start_kernel(long long n, const int* __restrict__ adj_ptr, const int* __restrict__ adj,
-                                    const int* __restrict__ elem, int n_el, const double* __restrict__ Ke,
-                                    const unsigned char* __restrict__ free_, const double* __restrict__ b,
-                                    const double* __restrict__ D, const double* __restrict__ x,
-                                    double* __restrict__ r, double* __restrict__ z, double* __restrict__ p,
-                                    double* __restrict__ part) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  double rz = 0.0, rr = 0.0;
-  if (i < n) {
-    double rx = 0.0, ry = 0.0, zx = 0.0, zy = 0.0;
-    if (free_[i] == 1) {
-      double kx, ky;
-      subpb2_gather_row(i, adj_ptr, adj, elem, n_el, Ke, x, kx, ky);
-      rx = b[2 * i] - kx;
-      ry = b[2 * i + 1] - ky;
-      zx = rx / D[i];
-      zy = ry / D[i];
+template <bool ONE>
+__global__ void __launch_bounds__(kCgThreads) subpb2_cg_kernel(
+    int start, int iters, long long n, const int* __restrict__ adj_ptr, const int* __restrict__ adj,
+    const int* __restrict__ elem, int n_el, const double* __restrict__ Ke, const unsigned char* __restrict__ free_,
+    const int* __restrict__ col, const double* __restrict__ val, const unsigned char* __restrict__ cnt,
+    const double* __restrict__ D, double* __restrict__ x, double2* __restrict__ r, double2* __restrict__ z,
+    double2* __restrict__ p0, double2* __restrict__ p1, double2* __restrict__ q, double2* __restrict__ parts,
+    double tol2, int maxit, Subpb2Scalars* sc) {
+  __shared__ double red[2 * (kCgThreads / 32)];
+  const long long stride = (long long)gridDim.x * kCgThreads, first = blockIdx.x * (long long)kCgThreads + threadIdx.x;
+  unsigned int epoch = 0;
+  double rz, rr0, beta = 0.0;
+  int it = 0;
+  if (start) {  // r = b - K x, z = r / D on the free nodes
+    double srz = 0.0, srr = 0.0;
+    for (long long i = first; i < n; i += stride) {
+      double2 ri = make_double2(0.0, 0.0), zi = ri;
+      if (free_[i] == 1) {
+        double kx = 0.0, ky = 0.0;
+        const int m = cnt[i];
+        if (m == kEllOverflow)
+          subpb2_gather_row(i, adj_ptr, adj, elem, n_el, Ke, x, kx, ky);
+        else
+          for (int k = 0; k < m; ++k) {
+            const long long c = col[k * n + i];
+            const double a = val[k * n + i];
+            kx = fma(a, x[2 * c], kx);
+            ky = fma(a, x[2 * c + 1], ky);
+          }
+        ri = make_double2(r[i].x - kx, r[i].y - ky);
+        zi = make_double2(ri.x / D[i], ri.y / D[i]);
+      }
+      r[i] = ri;
+      z[i] = zi;
+      p0[i] = p1[i] = q[i] = make_double2(0.0, 0.0);
+      srz += ri.x * zi.x + ri.y * zi.y;
+      srr += ri.x * ri.x + ri.y * ri.y;
     }
-    r[2 * i] = rx;
-    r[2 * i + 1] = ry;
-    z[2 * i] = zx;
-    z[2 * i + 1] = zy;
-    p[2 * i] = zx;
-    p[2 * i + 1] = zy;
-    rz = rx * zx + ry * zy;
-    rr = rx * rx + ry * ry;
+    if (!grid_exchange(parts, epoch, sc, srz, srr, red)) return;
+    rz = srz;
+    rr0 = srr;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      sc->rr0 = rr0;
+      sc->rz = rz;
+      sc->it = 0;
+      sc->ok = 1;
+      sc->done = rr0 == 0.0;
+    }
+    if (rr0 == 0.0) return;
+  } else {  // the last launch's state
+    rz = sc->rz;
+    rr0 = sc->rr0;
+    it = sc->it;
+    beta = sc->beta;
   }
-  block_partial(rz, rr, part);
-}
-
-__global__ void subpb2_init_scalars_kernel(const double* __restrict__ part, int nparts, Subpb2Scalars* sc) {
-  double rz, rr;
-  sum_partials(part, nparts, rz, rr);
-  if (threadIdx.x == 0) {
-    sc->rz = rz;
-    sc->rr0 = rr;
-    sc->rr = rr;
-    sc->it = 0;
-    sc->ok = 1;
-    sc->done = rr == 0.0 ? 1 : 0;
+  // ONE: the thread's node in registers
+  const long long i1 = first;
+  const bool mine = ONE && i1 < n && free_[i1] == 1;
+  const int m1 = mine ? cnt[i1] : 0;
+  int c1[kEllRegs];
+  double a1[kEllRegs], x1x = 0.0, x1y = 0.0, d1 = 1.0;
+  double2 r1 = make_double2(0.0, 0.0), z1 = r1, pa = r1;
+#pragma unroll
+  for (int k = 0; k < kEllRegs; ++k) {
+    const bool on = mine && m1 != kEllOverflow && k < m1;
+    c1[k] = on ? col[k * n + i1] : (mine ? (int)i1 : 0);
+    a1[k] = on ? val[k * n + i1] : 0.0;
   }
-}
-
-// q = K p on the free nodes (0 elsewhere) and the partial p . q.
-__global__ void subpb2_matvec_kernel(long long n, const int* __restrict__ adj_ptr, const int* __restrict__ adj,
-                                     const int* __restrict__ elem, int n_el, const double* __restrict__ Ke,
-                                     const unsigned char* __restrict__ free_, const double* __restrict__ p,
-                                     double* __restrict__ q, double* __restrict__ part,
-                                     const Subpb2Scalars* __restrict__ sc) {
-  if (sc->done) return;
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  double pq = 0.0;
-  if (i < n) {
-    double qx = 0.0, qy = 0.0;
-    if (free_[i] == 1) subpb2_gather_row(i, adj_ptr, adj, elem, n_el, Ke, p, qx, qy);
-    q[2 * i] = qx;
-    q[2 * i + 1] = qy;
-    pq = p[2 * i] * qx + p[2 * i + 1] * qy;
+  if (mine) {
+    x1x = x[2 * i1];
+    x1y = x[2 * i1 + 1];
+    d1 = D[i1];
+    r1 = r[i1];
+    z1 = z[i1];
+    pa = (it & 1 ? p1 : p0)[i1];
   }
-  block_partial(pq, 0.0, part);
-}
-
-__global__ void subpb2_alpha_kernel(const double* __restrict__ part, int nparts, Subpb2Scalars* sc) {
-  if (sc->done) return;
-  double pq, unused;
-  sum_partials(part, nparts, pq, unused);
-  if (threadIdx.x == 0) {
+  for (int k_ = 0; k_ < iters; ++k_) {
+    // q = K p with p = z + beta p_old
+    double2* po = it & 1 ? p1 : p0;
+    double2* pn = it & 1 ? p0 : p1;
+    double pq = 0.0, unused = 0.0;
+    double2 q1 = make_double2(0.0, 0.0);
+    for (long long i = first; i < n; i += stride) {
+      if (free_[i] != 1) continue;
+      const int m = ONE ? m1 : cnt[i];
+      const double2 zi = ONE ? z1 : z[i], pi = ONE ? pa : po[i];
+      const double2 pv = make_double2(fma(beta, pi.x, zi.x), fma(beta, pi.y, zi.y));
+      double qx = 0.0, qy = 0.0;
+      if (m == kEllOverflow) {
+        for (int a = adj_ptr[i]; a < adj_ptr[i + 1]; ++a) {
+          const int e = adj[a] >> 3;
+          const double* kr = Ke + (long long)e * 64 + (adj[a] & 7) * 8;
+          for (int b = 0; b < 8; ++b) {
+            const long long nb = elem[e + (long long)b * n_el] - 1;
+            if (nb < 0) continue;
+            const double2 zn = __ldcg(z + nb), pp = __ldcg(po + nb);
+            qx += kr[b] * fma(beta, pp.x, zn.x);
+            qy += kr[b] * fma(beta, pp.y, zn.y);
+          }
+        }
+      } else {
+        if constexpr (ONE) {
+          double2 zn[kEllRegs], pp[kEllRegs];
+#pragma unroll
+          for (int k = 0; k < kEllRegs; ++k) {  // entries past the row's end are the node's own, times 0
+            zn[k] = __ldcg(z + c1[k]);
+            pp[k] = __ldcg(po + c1[k]);
+          }
+#pragma unroll
+          for (int k = 0; k < kEllRegs; ++k) {
+            qx = fma(a1[k], fma(beta, pp[k].x, zn[k].x), qx);
+            qy = fma(a1[k], fma(beta, pp[k].y, zn[k].y), qy);
+          }
+        }
+#pragma unroll 4
+        for (int k = ONE ? kEllRegs : 0; k < m; ++k) {
+          const int c = col[k * n + i];
+          const double a = val[k * n + i];
+          const double2 zn = __ldcg(z + c), pp = __ldcg(po + c);
+          qx = fma(a, fma(beta, pp.x, zn.x), qx);
+          qy = fma(a, fma(beta, pp.y, zn.y), qy);
+        }
+      }
+      pn[i] = pv;
+      if (ONE) {
+        pa = pv;
+        q1 = make_double2(qx, qy);
+      } else {
+        q[i] = make_double2(qx, qy);
+      }
+      pq += pv.x * qx + pv.y * qy;
+    }
+    if (!grid_exchange(parts, epoch, sc, pq, unused, red)) return;
     if (!(pq > 0.0)) {  // no descent direction left: stop with what x holds
-      sc->done = 1;
-      sc->ok = 0;
-    } else {
-      sc->alpha = sc->rz / pq;
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc->done = 1;
+        sc->ok = 0;
+      }
+      break;
     }
-  }
-}
-
-// x += alpha p, r -= alpha q, z = r / D on the free nodes; partials r . z and r . r.
-__global__ void subpb2_update_kernel(long long n, const unsigned char* __restrict__ free_,
-                                     const double* __restrict__ D, const double* __restrict__ p,
-                                     const double* __restrict__ q, double* __restrict__ x, double* __restrict__ r,
-                                     double* __restrict__ z, double* __restrict__ part,
-                                     const Subpb2Scalars* __restrict__ sc) {
-  if (sc->done) return;
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  double rz = 0.0, rr = 0.0;
-  if (i < n && free_[i] == 1) {
-    const double al = sc->alpha;
-    for (int c = 0; c < 2; ++c) {
-      const long long k = 2 * i + c;
-      x[k] += al * p[k];
-      const double rn = r[k] - al * q[k];
-      r[k] = rn;
-      const double zn = rn / D[i];
-      z[k] = zn;
-      rz += rn * zn;
-      rr += rn * rn;
+    // x += alpha p, r -= alpha q, z = r / D on the free nodes
+    const double al = rz / pq;
+    double srz = 0.0, srr = 0.0;
+    for (long long i = first; i < n; i += stride) {
+      if (free_[i] != 1) continue;
+      const double2 pv = ONE ? pa : pn[i], qv = ONE ? q1 : q[i];
+      double2 rv = ONE ? r1 : r[i];
+      const double d = ONE ? d1 : D[i];
+      rv = make_double2(fma(-al, qv.x, rv.x), fma(-al, qv.y, rv.y));
+      const double2 zv = make_double2(rv.x / d, rv.y / d);
+      if (ONE) {
+        x1x = fma(al, pv.x, x1x);
+        x1y = fma(al, pv.y, x1y);
+        r1 = rv;
+        z1 = zv;
+      } else {
+        x[2 * i] = fma(al, pv.x, x[2 * i]);  // the caller's array: 8-byte aligned
+        x[2 * i + 1] = fma(al, pv.y, x[2 * i + 1]);
+        r[i] = rv;
+      }
+      z[i] = zv;
+      srz += rv.x * zv.x + rv.y * zv.y;
+      srr += rv.x * rv.x + rv.y * rv.y;
     }
+    if (!grid_exchange(parts, epoch, sc, srz, srr, red)) return;
+    beta = srz / rz;
+    rz = srz;
+    ++it;
+    const bool conv = srr <= tol2 * rr0, last = it >= maxit;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      sc->rz = rz;
+      sc->beta = beta;
+      sc->it = it;
+      if (conv || last) sc->done = 1;
+      if (last && !conv) sc->ok = 0;
+    }
+    if (conv || last) break;
   }
-  block_partial(rz, rr, part);
-}
-
-__global__ void subpb2_beta_kernel(const double* __restrict__ part, int nparts, double tol2, int maxit,
-                                   Subpb2Scalars* sc) {
-  if (sc->done) return;
-  double rz, rr;
-  sum_partials(part, nparts, rz, rr);
-  if (threadIdx.x == 0) {
-    sc->beta = rz / sc->rz;
-    sc->rz = rz;
-    sc->rr = rr;
-    sc->it += 1;
-    if (rr <= tol2 * sc->rr0 || sc->it >= maxit) sc->done = 1;
-    if (sc->it >= maxit && rr > tol2 * sc->rr0) sc->ok = 0;
+  if (mine) {
+    x[2 * i1] = x1x;
+    x[2 * i1 + 1] = x1y;
+    r[i1] = r1;
   }
 }
 
-// p = z + beta p (free nodes; p stays 0 elsewhere).  Runs after a converged step too: the
-// extra update leaves x untouched.
-__global__ void subpb2_direction_kernel(long long n, const unsigned char* __restrict__ free_,
-                                        const double* __restrict__ z, double* __restrict__ p,
-                                        const Subpb2Scalars* __restrict__ sc) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n || free_[i] != 1) return;
-  const double be = sc->beta;
-  p[2 * i] = z[2 * i] + be * p[2 * i];
-  p[2 * i + 1] = z[2 * i + 1] + be * p[2 * i + 1];
+int subpb2_cg_blocks(long long n) {
+  int dev = 0, sms = 148, per_sm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, subpb2_cg_kernel<false>, kCgThreads, 0);
+  int one = 1;  // both forms must fit: they take the same grid
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, subpb2_cg_kernel<true>, kCgThreads, 0);
+  // up to 3 CTAs an SM: enough loads in flight for large meshes, and short barriers
+  const long long most = (long long)sms * std::max(1, std::min(std::min(per_sm, one), 3)), need = (n + kCgThreads - 1) / kCgThreads;
+  return (int)std::max(1LL, std::min(most, need));
 }
-
-int subpb2_blocks(long long n) { return (int)((n + kSubpb2Threads - 1) / kSubpb2Threads); }
 
 int subpb2_mesh_tables(long long n, long long n_el, const int* E, long long n_dir, const int* dir,
                        std::vector<int>& ptr, std::vector<int>& adj, std::vector<unsigned char>& kind, char* msg,
@@ -454,41 +591,65 @@ int subpb2_mesh_tables(long long n, long long n_el, const int* E, long long n_di
 
 size_t subpb2_scalars_bytes() { return sizeof(Subpb2Scalars); }
 
-void subpb2_read_status(const void* host_copy, int* it, int* done, int* ok) {
+size_t subpb2_ell_bytes(long long n) { return (size_t)n * kEll * (sizeof(int) + sizeof(double)) + (size_t)n + 512; }
+
+void subpb2_read_status(const void* host_copy, int* it, int* done, int* ok, int* timeout) {
   const Subpb2Scalars* s = (const Subpb2Scalars*)host_copy;
   *it = s->it;
   *done = s->done;
   *ok = s->ok;
+  *timeout = s->timeout;
 }
+
+namespace {
+struct Ell {
+  double* val;
+  int* col;
+  unsigned char* cnt;
+};
+Ell ell_parts(void* base, long long n) {
+  Ell e;
+  e.val = (double*)base;
+  e.col = (int*)(e.val + (size_t)n * kEll);
+  e.cnt = (unsigned char*)(e.col + (size_t)n * kEll);
+  return e;
+}
+}  // namespace
 
 int launch_subpb2_setup(int n_el, const int* elem, const double* coords, long long n, const double* U,
                         const double* F, int order, double beta, double mu, double alpha, const int* adj_ptr,
-                        const int* adj, const unsigned char* free_, double* Ke, double* be, double* b, double* D,
-                        double* x, double* r, double* z, double* p, double* part, Subpb2Scalars* sc,
-                        cudaStream_t st) {
+                        const int* adj, const unsigned char* free_, double* Ke, double* be, void* ell, double* D,
+                        double* x, double* r, cudaStream_t st) {
   const long long rows = 8LL * n_el;
   subpb2_element_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, st>>>(n_el, elem, coords, n, U, F, order, beta, mu,
                                                                         alpha, Ke, be);
-  const int nb = subpb2_blocks(n);
-  subpb2_rhs_kernel<<<nb, kSubpb2Threads, 0, st>>>(n, adj_ptr, adj, Ke, be, free_, U, b, D, x);
-  subpb2_start_kernel<<<nb, kSubpb2Threads, 0, st>>>(n, adj_ptr, adj, elem, n_el, Ke, free_, b, D, x, r, z, p, part);
-  subpb2_init_scalars_kernel<<<1, kSubpb2Threads, 0, st>>>(part, nb, sc);
-  return 4;
+  const Ell e = ell_parts(ell, n);
+  subpb2_assemble_kernel<<<(unsigned)((n + kAsmThreads - 1) / kAsmThreads), kAsmThreads, 0, st>>>(
+      n, adj_ptr, adj, elem, n_el, Ke, be, free_, U, r, D, x, e.col, e.val, e.cnt);
+  return 2;
 }
 
-int launch_subpb2_iterations(int iters, int n_el, const int* elem, long long n, const int* adj_ptr, const int* adj,
-                             const double* Ke, const unsigned char* free_, const double* D, double* x, double* r,
-                             double* z, double* p, double* q, double* part, double tol2, int maxit,
-                             Subpb2Scalars* sc, cudaStream_t st) {
-  const int nb = subpb2_blocks(n);
-  for (int k = 0; k < iters; ++k) {
-    subpb2_matvec_kernel<<<nb, kSubpb2Threads, 0, st>>>(n, adj_ptr, adj, elem, n_el, Ke, free_, p, q, part, sc);
-    subpb2_alpha_kernel<<<1, kSubpb2Threads, 0, st>>>(part, nb, sc);
-    subpb2_update_kernel<<<nb, kSubpb2Threads, 0, st>>>(n, free_, D, p, q, x, r, z, part, sc);
-    subpb2_beta_kernel<<<1, kSubpb2Threads, 0, st>>>(part, nb, tol2, maxit, sc);
-    subpb2_direction_kernel<<<nb, kSubpb2Threads, 0, st>>>(n, free_, z, p, sc);
-  }
-  return 5 * iters;
+size_t subpb2_parts_bytes(int blocks) { return (size_t)blocks * 2 * sizeof(double2); }
+
+int launch_subpb2_cg(bool start, int iters, int blocks, long long n, const int* adj_ptr, const int* adj,
+                     const int* elem, int n_el, const double* Ke, const unsigned char* free_, void* ell,
+                     const double* D, double* x, double* r, double* z, double* p0, double* p1, double* q, void* parts,
+                     double tol2, int maxit, Subpb2Scalars* sc, cudaStream_t st) {
+  const Ell e = ell_parts(ell, n);
+  if (start)
+    cudaMemsetAsync(sc, 0, sizeof(Subpb2Scalars), st);
+  else
+    cudaMemsetAsync(&sc->arrived, 0, sizeof(unsigned int), st);  // barriers count from 1 in every launch
+  int s = start ? 1 : 0;
+  const int *col = e.col;
+  const double *val = e.val;
+  const unsigned char* cnt = e.cnt;
+  void* args[] = {&s, &iters, &n, &adj_ptr, &adj, &elem, &n_el, &Ke, &free_, &col, &val, &cnt, &D, &x, &r, &z, &p0,
+                  &p1, &q, &parts, &tol2, &maxit, &sc};
+  const void* k = n <= (long long)blocks * kCgThreads ? (const void*)subpb2_cg_kernel<true>
+                                                      : (const void*)subpb2_cg_kernel<false>;
+  cudaLaunchCooperativeKernel(k, dim3((unsigned)blocks), dim3(kCgThreads), args, 0, st);
+  return 1;
 }
 
 }  // namespace aldic
