@@ -96,8 +96,6 @@ struct Layout {
 };
 const Layout kL;
 
-__device__ __forceinline__ long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }
-
 // ------------------------------------------------------------------------- kernels
 // im2col of a 3 x 3, pad-1 convolution: row p = (b, oy, ox), column k = (ky, kx, ci), zero
 // outside the input and in the K padding.  Each thread writes 8 columns (one 16-byte store);
@@ -139,75 +137,126 @@ __global__ void im2col_kernel(const bf16* __restrict__ in, View v, bf16* __restr
 }
 
 // col2im (gather form, no atomics): the gradient of input pixel (b, iy, ix, ci) sums the
-// im2col gradient entries that read it.
-__global__ void col2im_kernel(const float* __restrict__ dA, float* __restrict__ dH, int batch, ConvI L) {
-  const long long total = (long long)batch * L.Hin * L.Win * L.Cin;
-  const int s = L.stride;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int ci = (int)(i % L.Cin);
-    const int ix = (int)((i / L.Cin) % L.Win);
-    const int iy = (int)((i / ((long long)L.Cin * L.Win)) % L.Hin);
-    const long long b = i / ((long long)L.Cin * L.Win * L.Hin);
-    float acc = 0.f;
+// im2col gradient entries that read it, in tap order.
+//
+// Bound by reading dA (95 MB for the deformed windows of a batch of 256).  Four channels a
+// thread (16-byte loads) and, with H, the ReLU of the layer below folded in (dZ = the sum where
+// H > 0, as BF16) instead of a pass over the FP32 gradient: 181 -> 52 us for that layer,
+// ReLU included.
+template <class Out>
+__device__ __forceinline__ float4 col2im_sum(const float* __restrict__ dA, const ConvI& L, long long b, int iy, int ix,
+                                             int ci) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int ky = 0; ky < 3; ++ky) {
-      const int ty = iy + 1 - ky;
-      if (ty < 0 || ty % s || ty / s >= L.Hout) continue;
+  for (int ky = 0; ky < 3; ++ky) {
+    const int ty = iy + 1 - ky;
+    if (ty < 0 || ty % L.stride || ty / L.stride >= L.Hout) continue;
 #pragma unroll
-      for (int kx = 0; kx < 3; ++kx) {
-        const int tx = ix + 1 - kx;
-        if (tx < 0 || tx % s || tx / s >= L.Wout) continue;
-        const long long p = (b * L.Hout + ty / s) * L.Wout + tx / s;
-        acc += dA[p * L.Kp + (ky * 3 + kx) * L.Cin + ci];
+    for (int kx = 0; kx < 3; ++kx) {
+      const int tx = ix + 1 - kx;
+      if (tx < 0 || tx % L.stride || tx / L.stride >= L.Wout) continue;
+      const long long p = (b * L.Hout + ty / L.stride) * L.Wout + tx / L.stride;
+      const Out v = *reinterpret_cast<const Out*>(dA + p * L.Kp + (ky * 3 + kx) * L.Cin + ci);
+      if constexpr (sizeof(Out) == 16) {
+        acc.x += v.x;
+        acc.y += v.y;
+        acc.z += v.z;
+        acc.w += v.w;
+      } else {
+        acc.x += v;
       }
     }
-    dH[i] = acc;
+  }
+  return acc;
+}
+
+__global__ void col2im_kernel(const float* __restrict__ dA, float* __restrict__ dH, int batch, ConvI L) {
+  const long long total = (long long)batch * L.Hin * L.Win * L.Cin;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int ci = (int)(i % L.Cin);
+    const long long pix = i / L.Cin;
+    const int ix = (int)(pix % L.Win), iy = (int)((pix / L.Win) % L.Hin);
+    dH[i] = col2im_sum<float>(dA, L, pix / ((long long)L.Win * L.Hin), iy, ix, ci).x;
+  }
+}
+
+// Cin a multiple of 4.
+__global__ void __launch_bounds__(256) col2im_relu_kernel(const float* __restrict__ dA, const bf16* __restrict__ H,
+                                                          bf16* __restrict__ dZ, int batch, ConvI L) {
+  const int groups = L.Cin / 4;
+  const long long total = (long long)batch * L.Hin * L.Win * groups;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int ci = (int)(i % groups) * 4;
+    const int pix = (int)(i / groups), row = pix / L.Win;
+    const uint2 h = *reinterpret_cast<const uint2*>(H + 4 * i);
+    const float4 g = col2im_sum<float4>(dA, L, row / L.Hin, row % L.Hin, pix % L.Win, ci);
+    const bf16* hb = reinterpret_cast<const bf16*>(&h);
+    __align__(8) bf16 o[4];
+    o[0] = __float2bfloat16_rn(__bfloat162float(hb[0]) > 0.f ? g.x : 0.f);
+    o[1] = __float2bfloat16_rn(__bfloat162float(hb[1]) > 0.f ? g.y : 0.f);
+    o[2] = __float2bfloat16_rn(__bfloat162float(hb[2]) > 0.f ? g.z : 0.f);
+    o[3] = __float2bfloat16_rn(__bfloat162float(hb[3]) > 0.f ? g.w : 0.f);
+    *reinterpret_cast<uint2*>(dZ + 4 * i) = *reinterpret_cast<const uint2*>(o);
   }
 }
 
 // Gradients of the correlation with the ReLU of its inputs folded in, over the whole conv2
 // output maps (zero on the ring outside the crops): dZR = dC fD / 32 where fR > 0 (B, 10, 10,
 // 32), dZD = dC^T fR / 32 where fD > 0 (B, 18, 18, 32), BF16; dC (B, 8, 8, 81) FP32.
-__global__ void corr_grad_ref_kernel(const float* __restrict__ dC, const bf16* __restrict__ fR,
-                                     const bf16* __restrict__ fD, bf16* __restrict__ dZR, long long total) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % 32);
-    const long long pix = i / 32;
-    const int x = (int)(pix % 10) - 1, y = (int)((pix / 10) % 10) - 1;  // crop coordinates
-    const long long b = pix / 100;
-    float s = 0.f;
-    if (x >= 0 && x < 8 && y >= 0 && y < 8 && __bfloat162float(fR[i]) > 0.f) {
-      const long long pos = (b * 8 + y) * 8 + x;
-      for (int d = 0; d < kDisp; ++d) {
-        const int di = d / 9 - 4, dj = d % 9 - 4;
-        s = fmaf(dC[pos * kDisp + d], __bfloat162float(fD[((b * 18 + y + 5 + di) * 18 + x + 5 + dj) * 32 + c]), s);
-      }
-    }
-    dZR[i] = __float2bfloat16_rn(s * (1.f / 32.f));
-  }
-}
+//
+// One CTA per sample: dC and both feature crops (57 KB) in shared memory, lanes = channels, so
+// a dC entry is one broadcast for a warp.  A thread per output reading all three from L2 took
+// 149 us a batch of 256 for the two gradients; this form 50 us.  Each sum runs over the
+// offsets in the same order.
+constexpr int kCorrGradThreads = 512;
+constexpr int kCorrGradSmem = (64 * kDisp + 256 * 32 + 64 * 32) * 4;
 
-__global__ void corr_grad_def_kernel(const float* __restrict__ dC, const bf16* __restrict__ fR,
-                                     const bf16* __restrict__ fD, bf16* __restrict__ dZD, long long total) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % 32);
-    const long long pix = i / 32;
-    const int q = (int)(pix % 18) - 1, p = (int)((pix / 18) % 18) - 1;  // crop coordinates
-    const long long b = pix / 324;
+__global__ void __launch_bounds__(kCorrGradThreads) corr_grad_kernel(const float* __restrict__ dC,
+                                                                    const bf16* __restrict__ fR,
+                                                                    const bf16* __restrict__ fD,
+                                                                    bf16* __restrict__ dZR, bf16* __restrict__ dZD) {
+  extern __shared__ float cg[];
+  float* c = cg;                 // [64][81]
+  float* D = c + 64 * kDisp;     // [16][16][32] the kept crop of fD
+  float* R = D + 256 * 32;       // [8][8][32] the kept crop of fR
+  const long long b = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kWarps = kCorrGradThreads / 32;
+  for (int i = tid; i < 64 * kDisp; i += kCorrGradThreads) c[i] = dC[b * 64 * kDisp + i];
+  for (int i = tid; i < 256 * 32; i += kCorrGradThreads)
+    D[i] = __bfloat162float(fD[((b * 18 + i / 512 + 1) * 18 + i / 32 % 16 + 1) * 32 + i % 32]);
+  for (int i = tid; i < 64 * 32; i += kCorrGradThreads)
+    R[i] = __bfloat162float(fR[((b * 10 + i / 256 + 1) * 10 + i / 32 % 8 + 1) * 32 + i % 32]);
+  __syncthreads();
+  for (int pix = warp; pix < 100; pix += kWarps) {
+    const int x = pix % 10 - 1, y = pix / 10 - 1;  // crop coordinates
     float s = 0.f;
-    if (p >= 0 && p < 16 && q >= 0 && q < 16 && __bfloat162float(fD[i]) > 0.f) {
-      for (int di = -4; di <= 4; ++di) {
-        const int ii = p - 4 - di;
-        if (ii < 0 || ii >= 8) continue;
-        for (int dj = -4; dj <= 4; ++dj) {
-          const int j = q - 4 - dj;
-          if (j < 0 || j >= 8) continue;
-          const long long rp = (b * 8 + ii) * 8 + j;
-          s = fmaf(dC[rp * kDisp + (di + 4) * 9 + (dj + 4)], __bfloat162float(fR[((b * 10 + ii + 1) * 10 + j + 1) * 32 + c]), s);
-        }
-      }
+    if (x >= 0 && x < 8 && y >= 0 && y < 8) {
+      const int pos = y * 8 + x;
+#pragma unroll 3
+      for (int di = 0; di < 9; ++di)
+#pragma unroll
+        for (int dj = 0; dj < 9; ++dj)
+          s = fmaf(c[pos * kDisp + di * 9 + dj], D[((y + di) * 16 + x + dj) * 32 + lane], s);
+      if (!(R[pos * 32 + lane] > 0.f)) s = 0.f;
     }
-    dZD[i] = __float2bfloat16_rn(s * (1.f / 32.f));
+    dZR[(b * 100 + pix) * 32 + lane] = __float2bfloat16_rn(s * (1.f / 32.f));
+  }
+  for (int pix = warp; pix < 324; pix += kWarps) {
+    const int q = pix % 18 - 1, p = pix / 18 - 1;  // crop coordinates
+    float s = 0.f;
+    if (p >= 0 && p < 16 && q >= 0 && q < 16) {
+      // the offsets (di, dj) whose reference position (p - 4 - di, q - 4 - dj) is in the crop
+      const int j0 = max(-4, q - 11), j1 = min(4, q - 4);
+      for (int di = max(-4, p - 11); di <= min(4, p - 4); ++di) {
+        const int base = (p - 4 - di) * 8 + q - 4;
+#pragma unroll 4
+        for (int dj = j0; dj <= j1; ++dj)
+          s = fmaf(c[(base - dj) * kDisp + (di + 4) * 9 + (dj + 4)], R[(base - dj) * 32 + lane], s);
+      }
+      if (!(D[(p * 16 + q) * 32 + lane] > 0.f)) s = 0.f;
+    }
+    dZD[(b * 324 + pix) * 32 + lane] = __float2bfloat16_rn(s * (1.f / 32.f));
   }
 }
 
@@ -660,18 +709,35 @@ __global__ void conv4_fold_kernel(const float* __restrict__ dWd, float* __restri
   }
 }
 
-// out[c, r] = in[r, c] (BF16, 32 x 32 tiles through shared memory)
-__global__ void transpose_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, long long R, long long Cn) {
-  __shared__ bf16 t[32][33];
-  const long long r0 = blockIdx.y * 32LL, c0 = blockIdx.x * 32LL;
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const long long r = r0 + j, c = c0 + threadIdx.x;
-    t[j][threadIdx.x] = (r < R && c < Cn) ? in[r * Cn + c] : __float2bfloat16_rn(0.f);
+// out[c, r] = in[r, c] (BF16), 64 x 64 tiles through shared memory, 16-byte loads and stores (R and
+// Cn multiples of 8: every matrix here; 32 x 32 tiles of 2-byte accesses took 205 us a training
+// step of 256, these 100 us).  A tile row holds 8 chunks of 8 columns.
+constexpr int kTrThreads = 256;
+__global__ void __launch_bounds__(kTrThreads) transpose_kernel(const bf16* __restrict__ in, bf16* __restrict__ out,
+                                                               long long R, long long Cn) {
+  // 2-byte entries at a pitch of 66: column reads of 8 rows by 32 lanes spread over the banks
+  __shared__ uint16_t t[64][66];
+  const long long r0 = blockIdx.y * 64LL, c0 = blockIdx.x * 64LL;
+#pragma unroll
+  for (int i = threadIdx.x; i < 512; i += kTrThreads) {
+    const int r = i >> 3, c = (i & 7) * 8;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (r0 + r < R && c0 + c < Cn) v = *reinterpret_cast<const uint4*>(in + (r0 + r) * Cn + c0 + c);
+    uint32_t* d = reinterpret_cast<uint32_t*>(&t[r][c]);
+    d[0] = v.x;
+    d[1] = v.y;
+    d[2] = v.z;
+    d[3] = v.w;
   }
   __syncthreads();
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const long long c = c0 + j, r = r0 + threadIdx.x;
-    if (c < Cn && r < R) out[c * R + r] = t[threadIdx.x][j];
+#pragma unroll
+  for (int i = threadIdx.x; i < 512; i += kTrThreads) {
+    const int c = i >> 3, r = (i & 7) * 8;
+    if (c0 + c >= Cn || r0 + r >= R) continue;
+    __align__(16) uint16_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = t[r + k][c];
+    *reinterpret_cast<uint4*>(out + (c0 + c) * R + r0 + r) = *reinterpret_cast<const uint4*>(v);
   }
 }
 
@@ -707,15 +773,55 @@ __global__ void mse_kernel(const float* __restrict__ Y, const float* __restrict_
   if (threadIdx.x == 0) atomicAdd(loss, red[0] / (float)(batch * kOut));
 }
 
-// db[c] += sum over rows of dZ[r, c] (each block sums a chunk of rows; one atomic per column)
-__global__ void bias_grad_kernel(const bf16* __restrict__ dZ, long long R, int Cn, float* __restrict__ db) {
-  const int c = threadIdx.x;
-  if (c >= Cn) return;
-  const long long per = ceil_div_ll(R, gridDim.x);
-  const long long r0 = blockIdx.x * per, r1 = r0 + per < R ? r0 + per : R;
+// db[c] += sum over rows of dZ[r, c] (Cn a multiple of 8, at most 128): each block sums a chunk of
+// rows, column by column in row order, with one atomic per column.
+//
+// The serial sum of a chunk (2 242 rows for conv1) is fixed, so its latency is what can be had: the
+// block brings tiles of rows to shared memory (16-byte loads, the next tile's in flight) and one
+// thread per column adds from there.  With one load in flight per column the eight launches of a
+// training step of 256 took 251 us (139 us for conv1's 331 776 rows), now 55 us.
+constexpr int kBiasThreads = 256, kBiasTile = 16384;  // bytes per tile
+__global__ void __launch_bounds__(kBiasThreads) bias_grad_kernel(const bf16* __restrict__ dZ, long long R, int Cn,
+                                                                 float* __restrict__ db) {
+  __shared__ __align__(16) unsigned char tile[kBiasTile];
+  constexpr int kPer = kBiasTile / 16 / kBiasThreads;  // 16-byte chunks per thread and tile
+  const long long per = (R + gridDim.x - 1) / gridDim.x, r0 = blockIdx.x * per;
+  const long long rows = r0 + per < R ? per : R - r0;
+  if (rows <= 0) return;
+  const int tid = threadIdx.x, trows = kBiasTile / (2 * Cn);
+  const uint4* src = reinterpret_cast<const uint4*>(dZ + r0 * Cn);
+  const long long chunks = rows * Cn / 8;
+  uint4 v[kPer];
+  auto fetch = [&](long long first) {
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const long long q = first + tid + k * kBiasThreads;
+      if (q < chunks) v[k] = src[q];
+    }
+  };
   float s = 0.f;
-  for (long long r = r0; r < r1; ++r) s += __bfloat162float(dZ[r * Cn + c]);
-  atomicAdd(db + c, s);
+  fetch(0);
+  for (long long t = 0; t < rows; t += trows) {
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) reinterpret_cast<uint4*>(tile)[tid + k * kBiasThreads] = v[k];
+    __syncthreads();
+    fetch((t + trows) * Cn / 8);
+    if (tid < Cn) {
+      const bf16* c = reinterpret_cast<const bf16*>(tile) + tid;
+      const int m = (int)(rows - t < trows ? rows - t : trows);
+      int r = 0;
+      for (; r + 16 <= m; r += 16) {
+        float x[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) x[k] = __bfloat162float(c[(r + k) * Cn]);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s += x[k];
+      }
+      for (; r < m; ++r) s += __bfloat162float(c[r * Cn]);
+    }
+  }
+  if (tid < Cn) atomicAdd(db + tid, s);
 }
 
 // Adam (Kingma & Ba 2015) on the flat FP32 parameters, refreshing their BF16 copies
@@ -865,8 +971,13 @@ int gemm(ProposalNet* net, const void* A, long long lda, const void* B, long lon
 }
 
 void transpose(ProposalNet* net, const bf16* in, bf16* out, long long R, long long Cn) {
-  const dim3 grid((unsigned)((Cn + 31) / 32), (unsigned)((R + 31) / 32));
-  transpose_kernel<<<grid, dim3(32, 8), 0, net->stream>>>(in, out, R, Cn);
+  const dim3 grid((unsigned)((Cn + 63) / 64), (unsigned)((R + 63) / 64));
+  transpose_kernel<<<grid, kTrThreads, 0, net->stream>>>(in, out, R, Cn);
+  ++net->launches;
+}
+
+void bias_grad(ProposalNet* net, const bf16* dZ, long long R, int Cn, float* db, int blocks = 148) {
+  bias_grad_kernel<<<blocks, kBiasThreads, 0, net->stream>>>(dZ, R, Cn, db);
   ++net->launches;
 }
 
@@ -963,21 +1074,23 @@ int conv_wgrad(ProposalNet* net, int i, int batch) {
   int rc = gemm(net, net->dZt[i], P, net->At[i], P, L.Cout, L.Kp, P, kEpiAtomic, net->g + kL.w[L.layer], nullptr,
                 nullptr, L.Kp, wsplit(L.Cout, L.Kp, P));
   if (rc) return rc;
-  bias_grad_kernel<<<148, L.Cout, 0, net->stream>>>(net->dZ[i], P, L.Cout, net->g + kL.b[L.layer]);
-  ++net->launches;
+  bias_grad(net, net->dZ[i], P, L.Cout, net->g + kL.b[L.layer]);
   return ALDIC_OK;
 }
 
 // gradient of convolution i's input: dA = dZ W, then col2im into net->dHf (FP32, the input's
-// NHWC layout)
-int conv_dgrad(ProposalNet* net, int i, int batch) {
+// NHWC layout) or, with H (the input, a ReLU's output), through that ReLU into dZ_in (BF16)
+int conv_dgrad(ProposalNet* net, int i, int batch, const bf16* H = nullptr, bf16* dZ_in = nullptr) {
   const ConvI& L = kConv[i];
   const long long P = P_of(i, batch);
   int rc = gemm(net, net->dZ[i], L.Cout, net->wt[L.layer], L.Cout, P, L.Kp, L.Cout, kEpiStore, net->dAf, nullptr,
                 nullptr, L.Kp, 1);
   if (rc) return rc;
   const long long nin = (long long)batch * L.Hin * L.Hin * L.Cin;
-  col2im_kernel<<<blocks_for(nin), 256, 0, net->stream>>>(net->dAf, net->dHf, batch, L);
+  if (H)
+    col2im_relu_kernel<<<blocks_for(nin / 4), 256, 0, net->stream>>>(net->dAf, H, dZ_in, batch, L);
+  else
+    col2im_kernel<<<blocks_for(nin), 256, 0, net->stream>>>(net->dAf, net->dHf, batch, L);
   ++net->launches;
   return ALDIC_OK;
 }
@@ -993,7 +1106,7 @@ int backward(ProposalNet* net, int batch, const bf16* X, const float* T) {
   const long long B = batch;
   NK(cudaMemsetAsync(net->g, 0, sizeof(float) * kL.n, st));
   NK(cudaMemsetAsync(net->loss, 0, sizeof(float), st));
-  mse_kernel<<<1, 256, 0, st>>>(net->Y, T, batch, net->dY, net->loss);
+  mse_kernel<<<(unsigned)((batch * kOutP + 255) / 256), 256, 0, st>>>(net->Y, T, batch, net->dY, net->loss);
   ++net->launches;
   // transposed weights for the data gradients (conv1's input needs none)
   for (int l = 1; l < 6; ++l) transpose(net, net->wb + kL.w[l], net->wt[l], kL.rows[l], kL.cols[l]);
@@ -1003,8 +1116,7 @@ int backward(ProposalNet* net, int batch, const bf16* X, const float* T) {
   int rc = gemm(net, net->dYt, B, net->Ht6, B, kOutP, kFcHid, B, kEpiAtomic, net->g + kL.w[5], nullptr, nullptr,
                 kFcHid, wsplit(kOutP, kFcHid, B));
   if (rc) return rc;
-  bias_grad_kernel<<<64, kOutP, 0, st>>>(net->dY, B, kOutP, net->g + kL.b[5]);
-  ++net->launches;
+  bias_grad(net, net->dY, B, kOutP, net->g + kL.b[5], 64);
   rc = gemm(net, net->dY, kOutP, net->wt[5], kOutP, B, kFcHid, kOutP, kEpiStore, net->dHf, nullptr, nullptr, kFcHid, 1);
   if (rc) return rc;
   relu_grad(net, net->H6, net->dZ6, B * kFcHid);
@@ -1014,8 +1126,7 @@ int backward(ProposalNet* net, int batch, const bf16* X, const float* T) {
   rc = gemm(net, net->dZt6, B, net->Ht5, B, kFcHid, kFcIn, B, kEpiAtomic, net->g + kL.w[4], nullptr, nullptr, kFcIn,
             wsplit(kFcHid, kFcIn, B));
   if (rc) return rc;
-  bias_grad_kernel<<<64, kFcHid, 0, st>>>(net->dZ6, B, kFcHid, net->g + kL.b[4]);
-  ++net->launches;
+  bias_grad(net, net->dZ6, B, kFcHid, net->g + kL.b[4], 64);
   rc = gemm(net, net->dZ6, kFcHid, net->wt[4], kFcHid, B, kFcIn, kFcHid, kEpiStore, net->dHf, nullptr, nullptr, kFcIn,
             1);
   if (rc) return rc;
@@ -1028,26 +1139,27 @@ int backward(ProposalNet* net, int batch, const bf16* X, const float* T) {
             kFcIn, 1);
   if (rc) return rc;
   conv4_fold_kernel<<<144, 256, 0, st>>>(net->dAf, net->g + kL.w[3]);
-  bias_grad_kernel<<<148, 64, 0, st>>>(net->dZ[kConv4], B * 16, 64, net->g + kL.b[3]);
-  net->launches += 2;
+  ++net->launches;
+  bias_grad(net, net->dZ[kConv4], B * 16, 64, net->g + kL.b[3]);
   rc = gemm(net, net->dZ[kConv4], kFcIn, net->W4dT, kFcIn, B, kFcIn, kFcIn, kEpiStore, net->dHf, nullptr, nullptr,
             kFcIn, 1);
   if (rc) return rc;
   relu_grad(net, net->H[kConv3], net->dZ[kConv3], B * 16 * 64);
   if ((rc = conv_wgrad(net, kConv3, batch)) || (rc = conv_dgrad(net, kConv3, batch))) return rc;
   // correlation: dHf holds dC (B, 8, 8, 81); the ReLUs of conv2's outputs folded in
-  corr_grad_ref_kernel<<<blocks_for(B * 100 * 32), 256, 0, st>>>(net->dHf, net->H[kConvR2], net->H[kConvD2],
-                                                                  net->dZ[kConvR2], B * 100 * 32);
-  corr_grad_def_kernel<<<blocks_for(B * 324 * 32), 256, 0, st>>>(net->dHf, net->H[kConvR2], net->H[kConvD2],
-                                                                  net->dZ[kConvD2], B * 324 * 32);
-  net->launches += 2;
+  NK(cudaFuncSetAttribute(corr_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCorrGradSmem));
+  corr_grad_kernel<<<(unsigned)B, kCorrGradThreads, kCorrGradSmem, st>>>(net->dHf, net->H[kConvR2], net->H[kConvD2],
+                                                                        net->dZ[kConvR2], net->dZ[kConvD2]);
+  ++net->launches;
   // conv2 and conv1 on the reference subset, then on the deformed window (shared weights)
-  if ((rc = conv_wgrad(net, kConvR2, batch)) || (rc = conv_dgrad(net, kConvR2, batch))) return rc;
-  relu_grad(net, net->H[kConvR1], net->dZ[kConvR1], B * 400 * 32);
+  if ((rc = conv_wgrad(net, kConvR2, batch)) ||
+      (rc = conv_dgrad(net, kConvR2, batch, net->H[kConvR1], net->dZ[kConvR1])))
+    return rc;
   im2col(net, kConvR1, batch, X, kViewRef);  // conv1 ran directly: its im2col rows for dW
   if ((rc = conv_wgrad(net, kConvR1, batch))) return rc;
-  if ((rc = conv_wgrad(net, kConvD2, batch)) || (rc = conv_dgrad(net, kConvD2, batch))) return rc;
-  relu_grad(net, net->H[kConvD1], net->dZ[kConvD1], B * 1296 * 32);
+  if ((rc = conv_wgrad(net, kConvD2, batch)) ||
+      (rc = conv_dgrad(net, kConvD2, batch, net->H[kConvD1], net->dZ[kConvD1])))
+    return rc;
   im2col(net, kConvD1, batch, X, kViewDef);
   return conv_wgrad(net, kConvD1, batch);
 }

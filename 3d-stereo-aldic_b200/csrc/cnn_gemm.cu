@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -44,8 +45,9 @@ struct GemmSmem {
   static constexpr int b_bytes = BN * kBK * 2;
   static constexpr int stage_bytes = a_bytes + b_bytes;
   static constexpr int bytes = kStages * stage_bytes + 1024;  // + 1024 for the alignment
-  static constexpr uint32_t acc_cols = BN < 32 ? 32 : BN;     // TMEM columns of one accumulator
-  static constexpr int per_sm = (227 * 1024) / bytes < 4 ? (227 * 1024) / bytes : 4;
+  static constexpr uint32_t acc_cols = BN < 32 ? 32 : BN == 96 ? 128 : BN;  // TMEM columns of one accumulator
+  // FP32 stores (kEpiStore) go through a 32 x 32 block per epilogue warp, rows 36 floats apart
+  static constexpr int store_bytes = 4 * 32 * 36 * 4;
 };
 
 struct TileGrid {
@@ -61,9 +63,46 @@ struct TileGrid {
 };
 
 template <int BN>
-__device__ __forceinline__ void gemm_epilogue_tile(const GemmEpi& epi, uint32_t tacc, int row, int n0, int M, int N) {
+__device__ __forceinline__ void gemm_epilogue_tile(const GemmEpi& epi, uint32_t tacc, int row, int n0, int M, int N,
+                                                   float* stage) {
+  int c_first = 0;
+  if constexpr (BN % 32 == 0) {
+    // FP32 stores of 32 whole columns: a row's 128 bytes are written by 8 consecutive lanes (16
+    // bytes a lane and a row a lane apart, the stores of conv2's data gradient took 82 us; so
+    // 27 us, in tiles of 96 columns)
+    const int lane = threadIdx.x & 31, row0 = row - lane;
+    if (epi.mode == kEpiStore && epi.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(epi.c32) & 15) == 0) {
 #pragma unroll 1
-  for (int c = 0; c < BN; c += 16) {
+      for (; c_first < BN && n0 + c_first + 32 <= N; c_first += 32) {
+        float v[32];
+        __syncwarp();
+        tmem_ld16(tacc + (uint32_t)c_first, *reinterpret_cast<float(*)[16]>(v));
+        tmem_ld16(tacc + (uint32_t)c_first + 16u, *reinterpret_cast<float(*)[16]>(v + 16));
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<float4*>(stage + lane * 36 + 4 * j) =
+              make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        __syncwarp();
+        const int col = n0 + c_first + (lane & 7) * 4;
+        float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (epi.bias) bias = make_float4(epi.bias[col], epi.bias[col + 1], epi.bias[col + 2], epi.bias[col + 3]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int r = j * 4 + (lane >> 3);
+          float4 q = *reinterpret_cast<const float4*>(stage + r * 36 + (lane & 7) * 4);
+          if (epi.bias) {
+            q.x += bias.x;
+            q.y += bias.y;
+            q.z += bias.z;
+            q.w += bias.w;
+          }
+          if (row0 + r < M) *reinterpret_cast<float4*>(epi.c32 + (size_t)(row0 + r) * epi.ldc + col) = q;
+        }
+      }
+    }
+  }
+#pragma unroll 1
+  for (int c = c_first; c < BN; c += 16) {
     float v[16];
     __syncwarp();  // tcgen05.ld is warp-collective: reconverge after the previous run's stores
     tmem_ld16(tacc + (uint32_t)c, v);
@@ -237,7 +276,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
       tcgen05_after_sync();
       gemm_epilogue_tile<BN>(epi, tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)b * kCols, m0 + q * 32 + lane,
-                             nt * BN, M, N);
+                             nt * BN, M, N,
+                             reinterpret_cast<float*>(smem + kStages * GemmSmem<BN>::stage_bytes) + q * 32 * 36);
       tcgen05_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[b]);
@@ -309,19 +349,22 @@ int launch_bn(const GemmArgs& g, cudaStream_t st) {
   tg.kb_total = kb_total;
   // persistent: as many CTAs as fit on the GPU at once (shared memory bound), at most one
   // per tile
-  const long long slots = (long long)num_sms() * GemmSmem<BN>::per_sm;
+  const int bytes = GemmSmem<BN>::bytes + (g.epi.mode == kEpiStore ? GemmSmem<BN>::store_bytes : 0);
+  const long long slots = (long long)num_sms() * std::min(4, (227 * 1024) / bytes);
   const int grid = (int)(tg.ntiles < slots ? tg.ntiles : slots);
   auto k = umma_gemm_kernel<BN>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::bytes);
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       GemmSmem<BN>::bytes + GemmSmem<BN>::store_bytes);
   cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  k<<<grid, kGemmThreads, GemmSmem<BN>::bytes, st>>>(ta, tb, g.epi, (int)g.M, (int)g.N, tg);
+  k<<<grid, kGemmThreads, bytes, st>>>(ta, tb, g.epi, (int)g.M, (int)g.N, tg);
   return 1;
 }
 
 }  // namespace
 
 // C = A * B^T (see GemmArgs); the BN tile is the smallest of 16, 32, 64, 128, 256 that holds
-// N (larger N take several column tiles of 256).  Returns the launch count, -1 on a layout
+// N.  Larger N take column tiles of 256, or of 96 where N fills those and would leave most of its
+// last tile of 256 empty (conv2's 288 columns: 3 x 96 instead of 256 + 32).  Returns the launch count, -1 on a layout
 // the tensor maps cannot describe.
 int launch_umma_gemm(const GemmArgs& g, cudaStream_t st) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0) return 0;
@@ -329,6 +372,7 @@ int launch_umma_gemm(const GemmArgs& g, cudaStream_t st) {
   if (g.N <= 32) return launch_bn<32>(g, st);
   if (g.N <= 64) return launch_bn<64>(g, st);
   if (g.N <= 128) return launch_bn<128>(g, st);
+  if (g.N > 256 && g.N % 96 == 0 && g.N % 256 != 0 && g.N % 256 <= 64) return launch_bn<96>(g, st);
   return launch_bn<256>(g, st);
 }
 
