@@ -55,7 +55,7 @@ struct aldic_ctx {
   double* I1 = nullptr;
   double* I2 = nullptr;
   double* iitot = nullptr;
-  size_t ii_cap = 0;
+  size_t ii_cap = 0, iitot_cap = 0;
   void* tscratch = nullptr;  // shared-product search scratch
   size_t tscratch_cap = 0;
   int warp_cap = kDefaultWarpCap;  // aldic_set_iteration_cap
@@ -477,12 +477,20 @@ static int search_common(aldic_ctx* c, const int* search, const int* gridx, cons
     CK(cudaStreamSynchronize(c->stream));
     if (c->I1) CK(cudaFree(c->I1));
     if (c->I2) CK(cudaFree(c->I2));
-    if (c->iitot) CK(cudaFree(c->iitot));
-    c->I1 = c->I2 = c->iitot = nullptr;
+    c->I1 = c->I2 = nullptr;
+    c->ii_cap = 0;
     CK(cudaMalloc(&c->I1, iin * sizeof(double)));
     CK(cudaMalloc(&c->I2, iin * sizeof(double)));
-    CK(cudaMalloc(&c->iitot, search_tot_bytes(c->M, c->N)));
     c->ii_cap = iin;
+  }
+  const size_t itot = search_tot_bytes(c->M, c->N);  // depends on the shape, not on the area alone
+  if (c->iitot_cap < itot) {
+    CK(cudaStreamSynchronize(c->stream));
+    if (c->iitot) CK(cudaFree(c->iitot));
+    c->iitot = nullptr;
+    c->iitot_cap = 0;
+    CK(cudaMalloc(&c->iitot, itot));
+    c->iitot_cap = itot;
   }
   // scratch for the tile kernel whenever one exists (the autotuner may choose either chunk)
   const size_t tbytes = list ? 0 : search_tile_bytes(c->M, c->N, winsize, step, nx, ny, search[0], search[1], 0);

@@ -29,6 +29,7 @@ namespace {
 
 constexpr int kTJ = 8;     // subset columns per tile
 constexpr int kRing = 128; // rows of the circular g buffer
+constexpr int kVB = 16;    // shift columns whose largest variance sum is kept as one
 
 // Smallest m >= n with m = 4 (mod 8): row strides of 128-bit loads across consecutive
 // rows then hit 8 distinct 16-byte bank groups per quarter warp.
@@ -88,6 +89,7 @@ struct TileScratch {
   float* cx;         // nx * ny x 2 NDA: products of the excluded template column
   int* best;         // nx * ny: crop index of the first maximum
   float* cf;         // one centring constant per tile
+  double* vb;        // MW x ceil(NW / kVB): largest V of every kVB consecutive columns
   double* rr;        // nx x 2 sides x 4 x (N+1): integral-image rows of the top / bottom ring windows
 };
 
@@ -110,7 +112,9 @@ inline size_t scratch_layout(int M, int N, int W1, int nx, int ny, int nda, char
   char* pb = take(n * sizeof(int));
   char* pf = take(n * sizeof(float));  // >= the number of tiles
   char* prr = take((size_t)nx * 8 * (size_t)(N + 1) * sizeof(double));
+  char* pvb = take(MW * ((NW + kVB - 1) / kVB) * sizeof(double));
   if (sc) {
+    sc->vb = (double*)pvb;
     sc->rr = (double*)prr;
     sc->cf = (float*)pf;
     sc->map = (float2*)pm;
@@ -129,33 +133,74 @@ __device__ __forceinline__ float rsqrt_from(double v) { return v > 0 ? (float)(1
 }  // namespace
 
 // Window mean and variance sum of g for every full (w+1)^2 window position (x, y) (top-left,
-// 0-based), with the same integral-image expression as window_sums.
-__global__ void window_map_kernel(const double* __restrict__ I1, const double* __restrict__ I2, int M, int N,
-                                  int W1, float2* __restrict__ map, double* __restrict__ V) {
-  const int MW = M - W1 + 1, NW = N - W1 + 1;
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= (long long)MW * NW) return;
-  const int x = (int)(p / NW), y = (int)(p % NW);  // row-major: consecutive shift columns adjacent
-  double S1, S2;
-  box_sums(x, x + W1 - 1, y, y + W1 - 1, I1, I2, (size_t)M + 1, &S1, &S2);
+// 0-based), with the same integral-image expression as window_sums; and, per x, the largest
+// variance sum of every kVB consecutive y (vb: MW x nvb), for window_rowmax_kernel.
+//
+// Bound by the 16 bytes a position written.  The integral images run along x and the maps along
+// y, so a tile of 32 x 32 positions goes through shared memory (one thread per position read the
+// integral images a column apart: 110 -> 33 us at 2048 x 2048).
+__global__ void __launch_bounds__(256) window_map_kernel(const double* __restrict__ I1, const double* __restrict__ I2,
+                                                         int M, int N, int W1, float2* __restrict__ map,
+                                                         double* __restrict__ V, double* __restrict__ vb) {
+  __shared__ double tv[32][33];
+  __shared__ float2 tm[32][33];
+  const int MW = M - W1 + 1, NW = N - W1 + 1, nvb = (NW + kVB - 1) / kVB;
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const double nwin = (double)W1 * W1;
-  const double v = S2 - S1 * S1 / nwin;
-  V[p] = v;
-  map[p] = make_float2((float)(S1 / nwin), rsqrt_from(v));
+  for (int k = ty; k < 32; k += 8) {  // lanes along x
+    const int x = x0 + tx, y = y0 + k;
+    double v = 0.0;
+    float2 m = make_float2(0.f, 0.f);
+    if (x < MW && y < NW) {
+      double S1, S2;
+      box_sums(x, x + W1 - 1, y, y + W1 - 1, I1, I2, (size_t)M + 1, &S1, &S2);
+      v = S2 - S1 * S1 / nwin;
+      m = make_float2((float)(S1 / nwin), rsqrt_from(v));
+    }
+    tv[k][tx] = v;
+    tm[k][tx] = m;
+  }
+  __syncthreads();
+  for (int k = ty; k < 32; k += 8) {  // lanes along y
+    const int x = x0 + k, y = y0 + tx;
+    if (x < MW && y < NW) {
+      V[(size_t)x * NW + y] = tv[tx][k];
+      map[(size_t)x * NW + y] = tm[tx][k];
+    }
+  }
+  if (ty < 32 / kVB && x0 + tx < MW && y0 + ty * kVB < NW) {  // positions outside the map are 0, as the maximum's start
+    double m = 0.0;
+#pragma unroll
+    for (int k = 0; k < kVB; ++k) m = fmax(m, tv[ty * kVB + k][tx]);
+    vb[(size_t)(x0 + tx) * nvb + y0 / kVB + ty] = m;
+  }
 }
 
-// H(x, j) = max(0, max over the non-ring shift columns db in [-U_j, D_j] of V(x, jj-1+db)).
-__global__ void window_rowmax_kernel(SearchArgs a, const double* __restrict__ V, double* __restrict__ H) {
-  const int W1 = a.winsize + 1, MW = a.M - W1 + 1, NW = a.N - W1 + 1;
+// H(x, j) = max(0, max over the non-ring shift columns db in [-U_j, D_j] of V(x, jj-1+db)), from
+// whole blocks of kVB positions and the single ones at the range's ends (146 -> 24 us for 40 000
+// subsets at radius 70).
+__global__ void window_rowmax_kernel(SearchArgs a, const double* __restrict__ V, const double* __restrict__ vb,
+                                     double* __restrict__ H) {
+  const int W1 = a.winsize + 1, MW = a.M - W1 + 1, NW = a.N - W1 + 1, nvb = (NW + kVB - 1) / kVB;
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= (long long)MW * a.ny) return;
-  const int x = (int)(p % MW), j = (int)(p / MW);
+  const int j = (int)(p % a.ny), x = (int)(p / a.ny);  // consecutive threads: overlapping ranges of one row
   const int jj = a.gy0 + j * a.step;
   const AxisGeom c = axis_geom(jj, a.winsize, a.s0, a.s1, a.N, a.gy1);
   double m = 0.0;
-  if (c.ok)
-    for (int db = -c.lo; db <= c.hi; ++db) m = fmax(m, V[(size_t)x * NW + (jj - 1 + db)]);
-  H[p] = m;
+  if (c.ok) {
+    const double* v = V + (size_t)x * NW;
+    const int y0 = jj - 1 - c.lo, y1 = jj - 1 + c.hi;  // inclusive
+    const int b0 = (y0 + kVB - 1) / kVB, b1 = (y1 + 1) / kVB;  // whole blocks [b0, b1)
+    if (b0 < b1) {
+      for (int y = y0; y < b0 * kVB; ++y) m = fmax(m, v[y]);
+      for (int b = b0; b < b1; ++b) m = fmax(m, vb[(size_t)x * nvb + b]);
+      for (int y = b1 * kVB; y <= y1; ++y) m = fmax(m, v[y]);
+    } else {
+      for (int y = y0; y <= y1; ++y) m = fmax(m, v[y]);
+    }
+  }
+  H[(size_t)x + (size_t)j * MW] = m;
 }
 
 // Rows r0 and r1 + 1 of both integral images for the top (a = 0) and bottom (a = na-1)
@@ -182,6 +227,9 @@ __global__ void ring_rows_kernel(SearchArgs a, double* __restrict__ rr) {
 // One warp per subset: template mean and norm, the window sums of the ring of partial
 // windows, the largest window variance sum over the crop (normxcorr2 zero threshold) and
 // validity; writes x, y and the NaN outputs of invalid subsets.
+//
+// Bound by the latency of its loads: the template's offsets are stepped (a division per sample took
+// 91 us for 15 600 subsets at window 32, now 79 us) and four loads are in flight.
 __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const double* __restrict__ H, const double* __restrict__ rr,
                                    SubsetPrm* __restrict__ prm, float2* __restrict__ ringv) {
   const int lane = threadIdx.x & 31;
@@ -201,14 +249,36 @@ __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const
   P.valid = 0;
   P.pad = 0;
   if (s.ok) {
+    // the template's mean, then its squared deviations; offsets stepped along the window
+    const float* tp = a.f + (s.ii - 1) + (size_t)(s.jj - 1) * a.M;
+    const int q_nt = 32 / W1, r_nt = 32 % W1, kstep = r_nt + q_nt * a.M, kwrap = a.M - W1;
+    const int aa0 = lane % W1, k0 = aa0 + lane / W1 * a.M;
     double sum = 0.0;
-    for (int p = lane; p < W1 * W1; p += 32)
-      sum += (double)a.f[(size_t)(s.ii - 1 + p % W1) + (size_t)(s.jj - 1 + p / W1) * a.M];
+    int aa = aa0, k = k0;
+#pragma unroll 4
+    for (int p = lane; p < W1 * W1; p += 32) {
+      sum += (double)tp[k];
+      aa += r_nt;
+      k += kstep;
+      if (aa >= W1) {
+        aa -= W1;
+        k += kwrap;
+      }
+    }
     const double fm = warp_sum(sum) / (double)(W1 * W1);
     double ss = 0.0;
+    aa = aa0;
+    k = k0;
+#pragma unroll 4
     for (int p = lane; p < W1 * W1; p += 32) {
-      const double d = (double)a.f[(size_t)(s.ii - 1 + p % W1) + (size_t)(s.jj - 1 + p / W1) * a.M] - fm;
+      const double d = (double)tp[k] - fm;
       ss += d * d;
+      aa += r_nt;
+      k += kstep;
+      if (aa >= W1) {
+        aa -= W1;
+        k += kwrap;
+      }
     }
     const double denT = sqrt(warp_sum(ss));
     if (denT != 0) {
@@ -262,10 +332,18 @@ __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const
 // rows of (f - cf) g at that column — the products a ring window drops.  f is centred by
 // the tile constant cf and g is zero outside the image, exactly as the tile kernel holds
 // them.
-__global__ void ring_column_kernel(SearchArgs a, const SubsetPrm* __restrict__ prm, int TI,
-                                   const float* __restrict__ tcf, float* __restrict__ cx) {
-  const int lane = threadIdx.x & 31;
-  const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+//
+// The column's f and g go to shared memory once; a lane then owns kRC consecutive shifts and slides
+// a register window of g along them (two loads and kRC FMAs a template row; the same sums in the
+// same order as a loop of two global loads per product, which took 359 us for 40 000 subsets at
+// radius 70 and takes 109 us so).
+constexpr int kRC = 4;
+constexpr int kRCMax = 512;  // shifts per pass: bounds the shared memory for any search radius
+__global__ void __launch_bounds__(128) ring_column_kernel(SearchArgs a, const SubsetPrm* __restrict__ prm, int TI,
+                                                          const float* __restrict__ tcf, float* __restrict__ cx) {
+  extern __shared__ float rc_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long t = blockIdx.x * 4LL + warp;
   const long long n = (long long)a.nx * a.ny;
   if (t >= n || !prm[t].valid) return;
   const int i = (int)(t % a.nx), j = (int)(t / a.nx);
@@ -273,22 +351,46 @@ __global__ void ring_column_kernel(SearchArgs a, const SubsetPrm* __restrict__ p
   const float cf = tcf[i / TI + (j / kTJ) * ((a.nx + TI - 1) / TI)];
   const int W1 = a.winsize + 1, DA0 = -a.s0 - 1, nda = a.s0 + a.s1 + 3;
   const int X = s.ii - 1, Y = s.jj - 1;
+  const int ng = (min(nda, kRCMax) + kRC - 1) / kRC * kRC + W1;  // g rows of a pass's padded shifts
+  float* fs = rc_smem + warp * (W1 + ng);
+  float* gs = fs + W1;
   float* out = cx + t * 2 * (long long)nda;
   for (int side = 0; side < 2; ++side) {
     const int c = Y + (side ? W1 - 1 : 0);
     const int cg = c + (side ? s.D + 1 : -s.U - 1);
-    for (int k = lane; k < nda; k += 32) {
-      const int aa = DA0 + k + s.L + 1;
-      if (aa < 0 || aa >= s.na) continue;
-      float acc = 0.f;
-      for (int r = 0; r < W1; ++r) {
-        const float fv = __ldg(a.f + (size_t)(X + r) + (size_t)c * a.M) - cf;
-        const int xg = X + r + DA0 + k;
-        float gv = 0.f;
-        if (xg >= 0 && xg < a.M && cg >= 0 && cg < a.N) gv = __ldg(a.g + (size_t)xg + (size_t)cg * a.M);
-        acc = fmaf(fv, gv, acc);
+    for (int r = lane; r < W1; r += 32) fs[r] = __ldg(a.f + (size_t)(X + r) + (size_t)c * a.M) - cf;
+    for (int b0 = 0; b0 < nda; b0 += kRCMax) {
+      for (int r = lane; r < ng; r += 32) {
+        const int xg = X + DA0 + b0 + r;
+        gs[r] = xg >= 0 && xg < a.M && cg >= 0 && cg < a.N ? __ldg(a.g + (size_t)xg + (size_t)cg * a.M) : 0.f;
       }
-      out[side * nda + k] = acc;
+      __syncwarp();
+      const int nb = min(nda - b0, kRCMax);
+      for (int k0 = lane * kRC; k0 < nb; k0 += 32 * kRC) {
+        float acc[kRC], w[kRC];
+#pragma unroll
+        for (int u = 0; u < kRC; ++u) {
+          acc[u] = 0.f;
+          w[u] = gs[k0 + u];
+        }
+        // w[(r + u) % kRC] = g of row r + k0 + u
+        for (int r0 = 0; r0 < W1; r0 += kRC) {
+#pragma unroll
+          for (int v = 0; v < kRC; ++v) {
+            if (r0 + v >= W1) break;
+            const float fv = fs[r0 + v];
+#pragma unroll
+            for (int u = 0; u < kRC; ++u) acc[u] = fmaf(fv, w[(v + u) % kRC], acc[u]);
+            w[v] = gs[k0 + kRC + r0 + v];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kRC; ++u) {
+          const int k = b0 + k0 + u, aa = DA0 + k + s.L + 1;
+          if (k0 + u < nb && aa >= 0 && aa < s.na) out[side * nda + k] = acc[u];
+        }
+      }
+      __syncwarp();
     }
   }
 }
@@ -1011,16 +1113,17 @@ int launch_search_tile(const SearchArgs& a, cudaStream_t st) {
   TileScratch sc;
   scratch_layout(a.M, a.N, W1, a.nx, a.ny, nda, (char*)a.tile_scratch, &sc);
   const long long n = (long long)a.nx * a.ny;
-  const long long npos = (long long)(a.M - W1 + 1) * (a.N - W1 + 1);
-  window_map_kernel<<<(unsigned)((npos + 255) / 256), 256, 0, st>>>(a.I1, a.I2, a.M, a.N, W1, sc.map, sc.V);
+  window_map_kernel<<<dim3((unsigned)((a.M - W1 + 32) / 32), (unsigned)((a.N - W1 + 32) / 32)), 256, 0, st>>>(
+      a.I1, a.I2, a.M, a.N, W1, sc.map, sc.V, sc.vb);
   const long long nh = (long long)(a.M - W1 + 1) * a.ny;
-  window_rowmax_kernel<<<(unsigned)((nh + 255) / 256), 256, 0, st>>>(a, sc.V, sc.H);
+  window_rowmax_kernel<<<(unsigned)((nh + 255) / 256), 256, 0, st>>>(a, sc.V, sc.vb, sc.H);
   const long long nrr = (long long)a.nx * 2 * (a.N + 1);
   ring_rows_kernel<<<(unsigned)((nrr + 255) / 256), 256, 0, st>>>(a, sc.rr);
   subset_prep_kernel<<<(unsigned)((n * 32 + 255) / 256), 256, 0, st>>>(a, sc.H, sc.rr, sc.prm, sc.ringv);
   const int ntiles = ((a.nx + e.TI - 1) / e.TI) * ((a.ny + kTJ - 1) / kTJ);
   tile_centre_kernel<<<(ntiles * 32 + 255) / 256, 256, 0, st>>>(a.nx, a.ny, e.TI, sc.prm, sc.cf);
-  ring_column_kernel<<<(unsigned)((n * 32 + 255) / 256), 256, 0, st>>>(a, sc.prm, e.TI, sc.cf, sc.cx);
+  const size_t rc_smem = 4 * (size_t)(W1 + (std::min(nda, kRCMax) + kRC - 1) / kRC * kRC + W1) * sizeof(float);
+  ring_column_kernel<<<(unsigned)((n + 3) / 4), 128, rc_smem, st>>>(a, sc.prm, e.TI, sc.cf, sc.cx);
   if (a.ev_start) cudaEventRecord(a.ev_start, st);
   if (e.launch(a, sc, st) != 0) return -1;
   if (a.ev_stop) cudaEventRecord(a.ev_stop, st);
