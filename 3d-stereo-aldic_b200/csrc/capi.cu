@@ -492,8 +492,8 @@ static int search_common(aldic_ctx* c, const int* search, const int* gridx, cons
     CK(cudaMalloc(&c->iitot, itot));
     c->iitot_cap = itot;
   }
-  // scratch for the tile kernel whenever one exists (the autotuner may choose either chunk)
-  const size_t tbytes = list ? 0 : search_tile_bytes(c->M, c->N, winsize, step, nx, ny, search[0], search[1], 0);
+  // scratch for the transforms or the tile kernel wherever the size allows one of them
+  const size_t tbytes = list ? 0 : search_scratch_bytes(c->M, c->N, winsize, step, nx, ny, search[0], search[1]);
   if (tbytes > c->tscratch_cap) {
     CK(cudaStreamSynchronize(c->stream));
     if (c->tscratch) CK(cudaFree(c->tscratch));
@@ -674,7 +674,7 @@ static int tune_search(aldic_ctx* c, SearchArgs& a) {
       int impl, chunk;
       const char* name;
     };
-    const Cand cands[] = {{1, 24, "tile24"}, {1, 16, "tile16"}, {2, 0, "direct"}};
+    const Cand cands[] = {{1, 24, "tile24"}, {1, 16, "tile16"}, {2, 0, "direct"}, {0, 0, "by_size"}};
     for (const Cand& cd : cands) {
       if (cd.impl == 1 && (!a.tile_scratch || !search_tile_available(a.step, a.winsize, cd.chunk))) continue;
       SearchArgs b = a;
@@ -696,7 +696,7 @@ static int tune_search(aldic_ctx* c, SearchArgs& a) {
           agree = (un || u0[i] == u1[i]) && (vn || v0[i] == v1[i]) && (pn || std::fabs(p0[i] - p1[i]) <= 1e-5);
         }
       first = false;
-      tn.ms.push_back({cd.name, agree ? ms : -ms});
+      if (cd.impl != 0) tn.ms.push_back({cd.name, agree ? ms : -ms});
       if (agree && ms < best) {
         best = ms;
         tn.a = cd.impl;
@@ -705,7 +705,7 @@ static int tune_search(aldic_ctx* c, SearchArgs& a) {
     }
     char ch[160];
     std::snprintf(ch, sizeof(ch), "{\"search\": \"%s\"}",
-                  tn.a == 2 ? "direct" : (tn.b == 16 ? "tile16" : "tile24"));
+                  tn.a == 0 ? "by_size" : tn.a == 2 ? "direct" : (tn.b == 16 ? "tile16" : "tile24"));
     tn.choice = ch;
     it = c->tuned.emplace(key, tn).first;
   }

@@ -95,12 +95,14 @@ struct SearchArgs {
   double* tot;  // row-pass chunk totals (scratch, search_tot_bytes)
   void* tile_scratch;  // shared-product search scratch (search_tile_bytes bytes), or null
   cudaEvent_t ev_start, ev_stop;  // recorded around the correlation kernel when non-null
-  int impl;   // 0: the shared-product tile kernel where one exists for (step, w + 1), else direct;
-              // 1: the tile kernel (falls back to direct without one); 2: the direct kernel
+  int impl;   // 0: transforms, the shared-product tile kernel (where one exists for (step, w + 1)) or the
+              // direct kernel, by size; 1: the tile kernel (direct without one); 2: the direct kernel
   int chunk;  // tile kernel shift columns per pass: 16 or 24 (0: the shape's default)
   const int* list;  // grid subsets (i + j nx) to search, or null for the whole grid; with a list
                     // the direct kernel runs and writes the outputs compactly (slot k = list[k])
   long long nlist;
+  const int* dlist = nullptr;   // direct kernel: the subsets to search (outputs in the grid's slots) and
+  const int* dcount = nullptr;  // their number, both on the device; null for the whole grid
 };
 // Whether a shared-product tile kernel exists for (step, w + 1) and fits this device.
 bool search_tile_available(int step, int winsize, int chunk);
@@ -135,6 +137,11 @@ int launch_subpb1(const Sub1Args& a, int wmax_x, int wmax_y, cudaStream_t st);
 size_t search_smem_bytes(int winsize, int s0, int s1);
 size_t search_tot_bytes(int M, int N);
 int launch_search(const SearchArgs& a, cudaStream_t st);
+int launch_search_direct(const SearchArgs& a, cudaStream_t st);  // the direct kernel alone
+bool search_direct_available(int winsize);
+// scratch of the tile kernel or the transforms, the larger; 0 where neither exists for the size
+size_t search_scratch_bytes(int M, int N, int winsize, int step, int nx, int ny, int s0, int s1);
+int launch_search_fft(const SearchArgs& a, cudaStream_t st);  // < 0: not for this call
 // Shared-product search (search_tile.cu): scratch size (0 when the step / window pair has
 // no tile kernel), and the launcher (returns the launch count, or -1 when not available).
 constexpr int kDefaultWarpCap = 8;   // default IcgnArgs / Sub1Args warp_cap

@@ -231,9 +231,9 @@ __global__ void __launch_bounds__(512, 1) ncc_search_kernel(SearchArgs a, int st
   const size_t ld = (size_t)a.M + 1;
   float* Tp = reinterpret_cast<float*>(smem_raw);
   float* Dt = Tp + TR * W1;
-  const long long n = a.list ? a.nlist : (long long)a.nx * a.ny;
+  const long long n = a.list ? a.nlist : a.dlist ? *a.dcount : (long long)a.nx * a.ny;
   for (long long q = blockIdx.x; q < n; q += gridDim.x) {
-    const long long t = a.list ? (long long)a.list[q] : q;
+    const long long t = a.list ? (long long)a.list[q] : a.dlist ? (long long)a.dlist[q] : q;
     const SubsetGeom s = subset_geom(a, t);
     const long long o = a.list ? q : subset_out(a, t);
     if (tid == 0) {
@@ -460,10 +460,21 @@ int launch_search(const SearchArgs& a, cudaStream_t st) {
   const long long n = a.list ? a.nlist : (long long)a.nx * a.ny;
   if (n <= 0) return 0;
   launch_integral(a.g, a.M, a.N, a.I1, a.I2, a.tot, st);
-  // shared products over tiles of subsets where a tile kernel exists for (step, w + 1) (a
-  // subset list takes the direct kernel)
+  // transforms, or shared products over tiles of subsets where a tile kernel exists for (step, w + 1)
+  // (a subset list takes the direct kernel)
+  const int fl = launch_search_fft(a, st);
+  if (fl >= 0) return 3 + fl;
   const int tl = a.list ? -1 : launch_search_tile(a, st);
   if (tl >= 0) return 3 + tl;
+  const int l = launch_search_direct(a, st);
+  return l < 0 ? l : 3 + l;
+}
+
+// The direct kernel's templates hold at most 120 rows.
+bool search_direct_available(int winsize) { return round_up8(winsize + 1) <= 120; }
+
+int launch_search_direct(const SearchArgs& a, cudaStream_t st) {
+  const long long n = a.list ? a.nlist : (long long)a.nx * a.ny;
   const int na = crop_max(a.s0, a.s1);
   const int sb = strip_columns(a.winsize, na, na, 200 * 1024);
   const SearchLayout L = search_layout(a.winsize, na, sb);
@@ -504,7 +515,7 @@ int launch_search(const SearchArgs& a, cudaStream_t st) {
     case 120: go(ncc_search_kernel<120>); break;
     default: return -1;
   }
-  return 4;
+  return 1;
 }
 
 }  // namespace aldic

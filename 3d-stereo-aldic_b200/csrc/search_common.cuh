@@ -101,7 +101,7 @@ struct SubsetPrm {
   double tolz;   // normxcorr2 zero threshold on the denominator
   double tolv;   // the same threshold on the window variance sum: (tolz / denT)^2
   int valid;     // geometry inside the image and a non-constant template
-  int pad;
+  float gnorm;   // transforms: norm of g over the cut-out window and the rows that share a transform with it
 };
 
 // FP64 NCC at crop shift (aa, bb) from its numerator sum((T - mean) D): the normxcorr2

@@ -22,6 +22,7 @@
 // products) from the window sum.  The argmax (first maximum in column-major crop order) is
 // refit in FP64 on the 3 x 3 neighbourhood, as the per-subset kernel does.
 #include "search_common.cuh"
+#include "search_fft.cuh"
 
 namespace aldic {
 
@@ -91,11 +92,14 @@ struct TileScratch {
   float* cf;         // one centring constant per tile
   double* vb;        // MW x ceil(NW / kVB): largest V of every kVB consecutive columns
   double* rr;        // nx x 2 sides x 4 x (N+1): integral-image rows of the top / bottom ring windows
+  void* rows;        // row spectra of the transforms
+  int* flist;        // nx * ny + 1: a count, then the subsets that the transforms leave to direct sums
 };
 
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-inline size_t scratch_layout(int M, int N, int W1, int nx, int ny, int nda, char* base, TileScratch* sc) {
+inline size_t scratch_layout(int M, int N, int W1, int nx, int ny, int nda, size_t row_bytes, char* base,
+                             TileScratch* sc) {
   const size_t MW = (size_t)(M - W1 + 1), NW = (size_t)(N - W1 + 1), n = (size_t)nx * ny;
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -113,7 +117,11 @@ inline size_t scratch_layout(int M, int N, int W1, int nx, int ny, int nda, char
   char* pf = take(n * sizeof(float));  // >= the number of tiles
   char* prr = take((size_t)nx * 8 * (size_t)(N + 1) * sizeof(double));
   char* pvb = take(MW * ((NW + kVB - 1) / kVB) * sizeof(double));
+  char* pl = take((n + 1) * sizeof(int));
+  char* pw = take(row_bytes);
   if (sc) {
+    sc->flist = (int*)pl;
+    sc->rows = pw;
     sc->vb = (double*)pvb;
     sc->rr = (double*)prr;
     sc->cf = (float*)pf;
@@ -130,32 +138,40 @@ inline size_t scratch_layout(int M, int N, int W1, int nx, int ny, int nda, char
 
 __device__ __forceinline__ float rsqrt_from(double v) { return v > 0 ? (float)(1.0 / sqrt(v)) : INFINITY; }
 
+// Whether a window's sum of squares is no more than the rounding of the integral image (its corner):
+// a window of zeros, as under a mask.  Its products are exactly zero, which a transform does not give.
+__device__ __forceinline__ bool is_zero(double S2, double corner) { return S2 <= 3.6e-15 * corner; }
+
 }  // namespace
 
-// Window mean and variance sum of g for every full (w+1)^2 window position (x, y) (top-left,
+// Window mean and variance sum of g (T float: 1 / sqrt of the variance sum alone) for every full (w+1)^2 window position (x, y) (top-left,
 // 0-based), with the same integral-image expression as window_sums; and, per x, the largest
 // variance sum of every kVB consecutive y (vb: MW x nvb), for window_rowmax_kernel.
 //
 // Bound by the 16 bytes a position written.  The integral images run along x and the maps along
 // y, so a tile of 32 x 32 positions goes through shared memory (one thread per position read the
 // integral images a column apart: 110 -> 33 us at 2048 x 2048).
+template <typename T>
 __global__ void __launch_bounds__(256) window_map_kernel(const double* __restrict__ I1, const double* __restrict__ I2,
-                                                         int M, int N, int W1, float2* __restrict__ map,
+                                                         int M, int N, int W1, T* __restrict__ map,
                                                          double* __restrict__ V, double* __restrict__ vb) {
   __shared__ double tv[32][33];
-  __shared__ float2 tm[32][33];
+  __shared__ T tm[32][33];
   const int MW = M - W1 + 1, NW = N - W1 + 1, nvb = (NW + kVB - 1) / kVB;
   const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const double nwin = (double)W1 * W1;
   for (int k = ty; k < 32; k += 8) {  // lanes along x
     const int x = x0 + tx, y = y0 + k;
     double v = 0.0;
-    float2 m = make_float2(0.f, 0.f);
+    T m{};
     if (x < MW && y < NW) {
       double S1, S2;
       box_sums(x, x + W1 - 1, y, y + W1 - 1, I1, I2, (size_t)M + 1, &S1, &S2);
       v = S2 - S1 * S1 / nwin;
-      m = make_float2((float)(S1 / nwin), rsqrt_from(v));
+      if constexpr (sizeof(T) == sizeof(float))
+        m = v <= 0 || is_zero(S2, I2[(size_t)(x + W1) + (size_t)(y + W1) * ((size_t)M + 1)]) ? 0.f : rsqrt_from(v);
+      else
+        m = make_float2((float)(S1 / nwin), rsqrt_from(v));
     }
     tv[k][tx] = v;
     tm[k][tx] = m;
@@ -225,13 +241,13 @@ __global__ void ring_rows_kernel(SearchArgs a, double* __restrict__ rr) {
 }
 
 // One warp per subset: template mean and norm, the window sums of the ring of partial
-// windows, the largest window variance sum over the crop (normxcorr2 zero threshold) and
-// validity; writes x, y and the NaN outputs of invalid subsets.
+// windows (zeros: 0 for the 1 / sqrt of a window of zeros), the largest window variance sum over the
+// crop (normxcorr2 zero threshold) and validity; writes x, y and the NaN outputs of invalid subsets.
 //
 // Bound by the latency of its loads: the template's offsets are stepped (a division per sample took
 // 91 us for 15 600 subsets at window 32, now 79 us) and four loads are in flight.
 __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const double* __restrict__ H, const double* __restrict__ rr,
-                                   SubsetPrm* __restrict__ prm, float2* __restrict__ ringv) {
+                                   bool zeros, SubsetPrm* __restrict__ prm, float2* __restrict__ ringv) {
   const int lane = threadIdx.x & 31;
   const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const long long n = (long long)a.nx * a.ny;
@@ -247,7 +263,7 @@ __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const
   SubsetPrm P;
   P.fm = P.denT = P.tolz = P.tolv = 0.0;
   P.valid = 0;
-  P.pad = 0;
+  P.gnorm = 0.f;
   if (s.ok) {
     // the template's mean, then its squared deviations; offsets stepped along the window
     const float* tp = a.f + (s.ii - 1) + (size_t)(s.jj - 1) * a.M;
@@ -301,7 +317,7 @@ __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const
           const double S2 = (R[3 * N1 + c1 + 1] - R[3 * N1 + c0]) - (R[2 * N1 + c1 + 1] - R[2 * N1 + c0]);
           const double v = S2 - S1 * S1 / nwin;
           m = fmax(m, v);
-          rv[side * nda + bb] = make_float2((float)(S1 / nwin), rsqrt_from(v));
+          rv[side * nda + bb] = make_float2((float)(S1 / nwin), zeros && (v <= 0 || is_zero(S2, R[3 * N1 + c1 + 1])) ? 0.f : rsqrt_from(v));
         }
       }
       for (int k = lane; k < 2 * s.na; k += 32) {
@@ -310,7 +326,8 @@ __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const
         window_sums(s, w, aa, side ? s.nb - 1 : 0, a.I1, a.I2, ld, &S1, &S2);
         const double v = S2 - S1 * S1 / nwin;
         m = fmax(m, v);
-        rv[(2 + side) * nda + aa] = make_float2((float)(S1 / nwin), rsqrt_from(v));
+        const size_t corner = (size_t)(min(s.dr1, s.dr0 - 1 + aa + w) + 1) + (size_t)(min(s.dc1, s.dc0 - 1 + (side ? s.nb - 1 : 0) + w) + 1) * ld;
+        rv[(2 + side) * nda + aa] = make_float2((float)(S1 / nwin), zeros && (v <= 0 || is_zero(S2, a.I2[corner])) ? 0.f : rsqrt_from(v));
       }
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
@@ -319,6 +336,11 @@ __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const
       P.tolz = sqrt(matlab_eps_d(denT * sqrt(fmax(m, 0.0))));
       P.tolv = (P.tolz / denT) * (P.tolz / denT);
       P.valid = 1;
+      if (zeros) {
+        double S1, S2;
+        box_sums(max(s.dr0 - 1, 0), min(s.dr1 + 1, a.M - 1), s.dc0, s.dc1, a.I1, a.I2, ld, &S1, &S2);
+        P.gnorm = (float)sqrt(S2);
+      }
     }
   }
   if (lane == 0) {
@@ -1004,6 +1026,7 @@ __global__ void __launch_bounds__(256, 3) subset_refit_kernel(SearchArgs a, cons
   if (!P.valid) return;
   const SubsetGeom s = subset_geom(a, t);
   const int bi = best[t];
+  if (bi < 0) return;  // left to direct sums
   refit_peak_warp(a, s, subset_out(a, t), bi % s.na, bi / s.na, P.fm, P.denT, P.tolz);
 }
 
@@ -1101,7 +1124,50 @@ size_t search_tile_bytes(int M, int N, int winsize, int step, int nx, int ny, in
   const int W1 = winsize + 1;
   TileEntry e;
   if (!tile_entry(step, W1, chunk, &e) || M < W1 || N < W1 || nx <= 0 || ny <= 0) return 0;
-  return scratch_layout(M, N, W1, nx, ny, s0 + s1 + 3, nullptr, nullptr);
+  return scratch_layout(M, N, W1, nx, ny, s0 + s1 + 3, 0, nullptr, nullptr);
+}
+
+size_t search_tables_bytes(const SearchArgs& a, size_t row_bytes) {
+  return scratch_layout(a.M, a.N, a.winsize + 1, a.nx, a.ny, a.s0 + a.s1 + 3, row_bytes, nullptr, nullptr);
+}
+
+// The waves of tiles times their products and shifts: a fit to measured times, see search_fft.cu.
+double search_tile_us(const SearchArgs& a) {
+  const int W1 = a.winsize + 1, nda = a.s0 + a.s1 + 3;
+  TileEntry e;
+  if (!tile_entry(a.step, W1, a.chunk, &e) || !e.fits()) return -1;
+  const double fr = (e.TI - 1) * a.step + W1, fc = (kTJ - 1) * a.step + W1;
+  const double tiles = (double)((a.nx + e.TI - 1) / e.TI) * ((a.ny + kTJ - 1) / kTJ);
+  return ceil(tiles / 148) * fr * fc * nda * ((nda + 23) / 24 * 24) * 1.5e-5;
+}
+
+// The tables that both ways read.  zeros: for the transforms.
+static void launch_tables(const SearchArgs& a, const TileScratch& sc, bool zeros, cudaStream_t st) {
+  const int W1 = a.winsize + 1;
+  const long long n = (long long)a.nx * a.ny;
+  const dim3 mgrid((unsigned)((a.M - W1 + 32) / 32), (unsigned)((a.N - W1 + 32) / 32));
+  if (zeros)
+    window_map_kernel<float><<<mgrid, 256, 0, st>>>(a.I1, a.I2, a.M, a.N, W1, (float*)sc.map, sc.V, sc.vb);
+  else
+    window_map_kernel<float2><<<mgrid, 256, 0, st>>>(a.I1, a.I2, a.M, a.N, W1, sc.map, sc.V, sc.vb);
+  const long long nh = (long long)(a.M - W1 + 1) * a.ny;
+  window_rowmax_kernel<<<(unsigned)((nh + 255) / 256), 256, 0, st>>>(a, sc.V, sc.vb, sc.H);
+  const long long nrr = (long long)a.nx * 2 * (a.N + 1);
+  ring_rows_kernel<<<(unsigned)((nrr + 255) / 256), 256, 0, st>>>(a, sc.rr);
+  subset_prep_kernel<<<(unsigned)((n * 32 + 255) / 256), 256, 0, st>>>(a, sc.H, sc.rr, zeros, sc.prm, sc.ringv);
+}
+
+int launch_search_tables(const SearchArgs& a, size_t row_bytes, SearchTables* t, cudaStream_t st) {
+  TileScratch sc;
+  scratch_layout(a.M, a.N, a.winsize + 1, a.nx, a.ny, a.s0 + a.s1 + 3, row_bytes, (char*)a.tile_scratch, &sc);
+  launch_tables(a, sc, true, st);
+  *t = SearchTables{(const float*)sc.map, sc.prm, sc.ringv, sc.best, sc.flist, sc.rows};
+  return 4;
+}
+
+void launch_search_refit(const SearchArgs& a, const SearchTables& t, cudaStream_t st) {
+  const long long n = (long long)a.nx * a.ny;
+  subset_refit_kernel<<<(unsigned)((n * 32 + 255) / 256), 256, 0, st>>>(a, t.prm, t.best);
 }
 
 int launch_search_tile(const SearchArgs& a, cudaStream_t st) {
@@ -1111,15 +1177,9 @@ int launch_search_tile(const SearchArgs& a, cudaStream_t st) {
     return -1;
   const int nda = a.s0 + a.s1 + 3;
   TileScratch sc;
-  scratch_layout(a.M, a.N, W1, a.nx, a.ny, nda, (char*)a.tile_scratch, &sc);
+  scratch_layout(a.M, a.N, W1, a.nx, a.ny, nda, 0, (char*)a.tile_scratch, &sc);
   const long long n = (long long)a.nx * a.ny;
-  window_map_kernel<<<dim3((unsigned)((a.M - W1 + 32) / 32), (unsigned)((a.N - W1 + 32) / 32)), 256, 0, st>>>(
-      a.I1, a.I2, a.M, a.N, W1, sc.map, sc.V, sc.vb);
-  const long long nh = (long long)(a.M - W1 + 1) * a.ny;
-  window_rowmax_kernel<<<(unsigned)((nh + 255) / 256), 256, 0, st>>>(a, sc.V, sc.vb, sc.H);
-  const long long nrr = (long long)a.nx * 2 * (a.N + 1);
-  ring_rows_kernel<<<(unsigned)((nrr + 255) / 256), 256, 0, st>>>(a, sc.rr);
-  subset_prep_kernel<<<(unsigned)((n * 32 + 255) / 256), 256, 0, st>>>(a, sc.H, sc.rr, sc.prm, sc.ringv);
+  launch_tables(a, sc, false, st);
   const int ntiles = ((a.nx + e.TI - 1) / e.TI) * ((a.ny + kTJ - 1) / kTJ);
   tile_centre_kernel<<<(ntiles * 32 + 255) / 256, 256, 0, st>>>(a.nx, a.ny, e.TI, sc.prm, sc.cf);
   const size_t rc_smem = 4 * (size_t)(W1 + (std::min(nda, kRCMax) + kRC - 1) / kRC * kRC + W1) * sizeof(float);

@@ -355,9 +355,10 @@ int aldic_measure_fp32_peak(aldic_ctx* ctx, double* tflops);
  *                            enough; 0 (default): they gather from the image through L1;
  *   ALDIC_OPT_SLOW_WARPS     warps per subset of the pass that continues the subsets still
  *                            iterating after the iteration cap: 2 (default) or 4;
- *   ALDIC_OPT_SEARCH_IMPL    aldic_integer_search: 0 (default) the shared-product tile kernel
- *                            where one is compiled for (step, winsize + 1), else the direct
- *                            per-subset correlation; 1 the tile kernel; 2 the direct kernel;
+ *   ALDIC_OPT_SEARCH_IMPL    aldic_integer_search: 0 (default) by size: correlation by FFTs,
+ *                            the shared-product tile kernel where one is compiled for
+ *                            (step, winsize + 1), or the direct per-subset correlation;
+ *                            1 the tile kernel (direct without one); 2 the direct kernel;
  *   ALDIC_OPT_SEARCH_CHUNK   shift columns per pass of the tile kernel: 16, 24 or 0 (the
  *                            shape's default);
  *   ALDIC_OPT_AUTOTUNE       1: the first call of every call shape (IC-GN: variant, winsize, n
