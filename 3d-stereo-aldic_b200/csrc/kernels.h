@@ -45,7 +45,7 @@ struct IcgnArgs {
   double band;   // relative margin around tol, added to the FP32 noise of |b|, within which an
                  // FP32 convergence test is re-decided by an FP64 re-solve of the subset (0: never)
   double noise;  // factor of the FP32 noise estimate of |b| added to the band
-  int staging;   // 1: the warp passes stage the deformed window by TMA when they can; 0: gathers
+  int staging;   // 1: the warp passes stage every deformed window that fits; 0: where enough fit an SM
   int slow_nw;   // warps per subset of the FP32 pass that continues the slow subsets: 2 or 4
   const double* F0;  // 4n initial displacement gradients [F11 F21 F12 F22] or null (the reference's 0)
   int slow_fp64; // 1: subsets still iterating after warp_cap are re-solved in FP64 (not the epipolar

@@ -12,10 +12,10 @@
 //
 // Work per subset and why it is taken: a direct sum costs na nb (w+1)^2 products (34 M at
 // radius 70 and window 41), the shared products of a tile 187 na nb = 3.8 M, the transforms about
-// 2.4 M operations.  40 000 subsets of that shape: 15.5 ms with the tile kernel, 9.5 ms so; 2088 of
-// window 33 at radius 20 705 us with the direct kernel, 257 us so (whole searches).  Bound by issue
-// slots and the latencies between the passes' barriers: one CTA of 16 warps fills an SM's shared
-// memory at L = 192.
+// 2.4 M operations.  40 000 subsets of that shape: 15.5 ms with the tile kernel, 8.2 ms so; 2088 of
+// window 33 at radius 20 705 us with the direct kernel, 255 us so (whole searches).  Bound by issue
+// slots (46 % used) and the latencies between the passes' barriers: one CTA of 12 warps fills an
+// SM's shared memory at L = 192.
 #include "search_common.cuh"
 #include "search_fft.cuh"
 
@@ -151,14 +151,15 @@ __device__ __forceinline__ void dft(float2 (&v)[N]) {
 }
 
 // A transform of L = 16 B values: 16-point DFTs of the elements a B + b (a = 0 .. 15), twiddled,
-// then B-point DFTs over b give the elements k1 + 16 k2.  Threads: the column product (8 items a
-// column) in two rounds.
+// then B-point DFTs over b give the elements k1 + 16 k2.
 template <int L>
 struct FftShape {
   static constexpr int B = L / 16, NU = L / 2 + 1;
-  // L = 192: as many warps as 128 registers allow; one CTA an SM in any case
-  static constexpr int NT = L == 192 ? 512 : (NU * 4 + 31) / 32 * 32;
-  static constexpr int MINB = L >= 160 ? 1 : L >= 128 ? 2 : L == 96 ? 3 : L == 80 ? 4 : L == 64 ? 5 : 6;
+  // threads and CTAs an SM: measured over both for every size (40 000 subsets at L = 192: 512 threads
+  // of 128 registers 9.48, 480 8.98, 384 of 168 8.18 ms; L = 80: 256 threads twice 1.13, 192 three
+  // times 0.99 ms)
+  static constexpr int NT = L >= 160 ? 384 : L == 144 ? 320 : L >= 96 ? 256 : L == 80 ? 192 : L == 64 ? 160 : 128;
+  static constexpr int MINB = L >= 160 ? 1 : L >= 96 ? 2 : L == 80 ? 3 : L == 64 ? 4 : 6;
   static_assert(L % 16 == 0 && L <= 192, "16 B with B <= 12");
 };
 
@@ -584,7 +585,7 @@ static int transform_size(int winsize, int s0, int s1) {
 // its shifts and template rounded up to its blocks; the factors (us) are fits to the measured times
 // of the three over windows of 21 to 49, steps of 8 to 32 and radii of 4 to 70, 55 us being what
 // the tables of the transforms' way cost at least (direct / transforms: 100 subsets at window 41 and
-// radius 5 97 / 108 us, 2088 at window 33 and radius 20 705 / 257 us; tile / transforms: 9604 at
+// radius 5 97 / 108 us, 2088 at window 33 and radius 20 705 / 255 us; tile / transforms: 9604 at
 // window 41, step 10 and radius 20 682 / 802 us, radius 35 1576 / 1106 us).
 static int transform_for(const SearchArgs& a) {
   const int W1 = a.winsize + 1, nda = a.s0 + a.s1 + 3;

@@ -139,6 +139,18 @@ def tile_flops(M, N, w, step, s0, s1):
     return 2.0 * FR * FC * nd * nd * tiles
 
 
+def transform_flops(M, N, w, step, s0, s1):
+    """FLOPs of the search's correlation by FFTs (5 L log2 L per complex transform of length L, two
+    real rows in one): the rows of g once per grid column; per subset the rows of T, the columns of
+    T, D and the product back, and the rows of the crop.  The products and the normalisation are
+    not counted."""
+    L = min(v for v in (48, 64, 80, 96, 128, 144, 160, 192) if v >= s0 + s1 + 3 + w - 1)
+    nx = len(range(1, M - w - step + 1, step))
+    ny = len(range(1, N - w - step + 1, step))
+    per = (w + 1) / 2 + 3 * (L / 2 + 1) + (s0 + s1 + 3) / 2
+    return 5.0 * L * np.log2(L) * (nx * ny * per + ny * M / 2)
+
+
 # ----------------------------------------------------------------------------------
 # clocks sampling during the timed region
 # ----------------------------------------------------------------------------------
@@ -1045,7 +1057,10 @@ def run_stereo(args, P, emit=True):
     pipe.icgn_events = None
     icgn_work = icgn_flops(pipe.buf["S"]["conv"].cpu().numpy(), P["w"])
     search_ms = prof_ms / max(prof_n, 1)
-    flops = tile_flops(P["size"], P["size"], P["w"], P["step"], P["s_stereo"], P["s_stereo"])
+    tuned = [t["choice"]["search"] for k, t in cS.tuning_report().items() if k.startswith("search")]
+    by_fft = all(t == "by_size" for t in tuned)  # the default choice, at this size the transforms
+    flops = (transform_flops if by_fft else tile_flops)(P["size"], P["size"], P["w"], P["step"], P["s_stereo"],
+                                                         P["s_stereo"])
     direct_flops = crop_flops(P["size"], P["size"], P["w"], P["step"], P["s_stereo"], P["s_stereo"])
     fp32_peak = measure_fp32_peak(torch, dev)
 
@@ -1101,15 +1116,16 @@ def run_stereo(args, P, emit=True):
                        "l2_flush": "inputs (4 x 8 MiB frames + 3 contexts of FP32 images/gradients/integral images) "
                                    "exceed the 126 MB L2 across a step", **P},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "fp32", "kernel": "ncc_tile_kernel (stereo integer search, shared products)",
+            "roofline": {"bound": "fp32", "kernel": "fft_rows_kernel + ncc_fft_kernel (stereo integer search, transforms)"
+                         if by_fft else "ncc_tile_kernel (stereo integer search, shared products)",
                          "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                          "frac": achieved / fp32_peak if fp32_peak else None,
-                         "traffic": TILE_TRAFFIC.get(args.workload), "traffic_unit": "bytes per launch",
+                         "traffic": None if by_fft else TILE_TRAFFIC.get(args.workload), "traffic_unit": "bytes per launch",
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel "
                                            "at this workload (separate capture)",
                          "peak_source": "measured on this GPU: the faster of a scalar FFMA and a packed FFMA2 "
                                         "loop (MEASURED_PEAKS.json holds only HBM and bf16 tensor peaks)",
-                         "algorithmic_flops_per_launch": flops, "flops_counted": "products only (2 per f*g)",
+                         "algorithmic_flops_per_launch": flops, "flops_counted": "5 L log2 L per transform" if by_fft else "products only (2 per f*g)",
                          "direct_correlation_flops": direct_flops, "launch_ms": search_ms,
                          "launches_timed": prof_n},
             "roofline_icgn": {"bound": "fp32", "kernel": "stereo IC-GN call (classify, one-warp pass, slow-subset "

@@ -350,9 +350,8 @@ int aldic_measure_fp32_peak(aldic_ctx* ctx, double* tflops);
  * beyond FP32 summation order, and with the FP64 re-solve not at all in the codes):
  *   ALDIC_OPT_ITERATION_CAP  as aldic_set_iteration_cap (1..1000, default 8);
  *   ALDIC_OPT_STAGING        1: the IC-GN warp passes stage each subset's deformed window in
- *                            shared memory by TMA 2-D tile loads when the image layout allows
- *                            (rows a multiple of 4, 16-byte aligned) and the window is small
- *                            enough; 0 (default): they gather from the image through L1;
+ *                            shared memory wherever its buffers fit; 0 (default): only where
+ *                            enough of them fit an SM, else they gather from the image;
  *   ALDIC_OPT_SLOW_WARPS     warps per subset of the pass that continues the subsets still
  *                            iterating after the iteration cap: 2 (default) or 4;
  *   ALDIC_OPT_SEARCH_IMPL    aldic_integer_search: 0 (default) by size: correlation by FFTs,
@@ -383,8 +382,8 @@ int aldic_measure_fp32_peak(aldic_ctx* ctx, double* tflops);
 #define ALDIC_OPT_SLOW_FP64 6
 #define ALDIC_OPT_FP64_THREADS 7
 /* Read-only statistics of the last aldic_local_icgn (aldic_get_option; waits for the call):
- * subsets re-solved in FP64, and 1 if a staging load outlasted its wait (the warp group then
- * gathered from the image). */
+ * subsets re-solved in FP64, and 1 if a staging load outlasted its wait (0: its loads do not wait
+ * on a barrier). */
 #define ALDIC_STAT_FP64_RESOLVES 100
 #define ALDIC_STAT_STAGING_TIMEOUT 101
 int aldic_set_option(aldic_ctx* ctx, int option, int value);
