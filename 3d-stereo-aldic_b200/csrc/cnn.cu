@@ -705,7 +705,7 @@ __global__ void conv4_fold_kernel(const float* __restrict__ dWd, float* __restri
         acc += dWd[(size_t)((oy * 4 + ox) * 64 + co) * 1024 + (iy * 4 + ix) * 64 + ci];
       }
     }
-    g[e] += acc;
+    g[e] = acc;
   }
 }
 
@@ -748,33 +748,38 @@ __global__ void relu_grad_kernel(const float* __restrict__ dH, const bf16* __res
     dZ[i] = __float2bfloat16_rn(__bfloat162float(H[i]) > 0.f ? dH[i] : 0.f);
 }
 
-// loss = mean over batch x 6 of (y - t)^2; dY = d loss / dy (BF16, the 6 outputs of 16 columns)
-__global__ void mse_kernel(const float* __restrict__ Y, const float* __restrict__ T, int batch, bf16* __restrict__ dY,
-                           float* __restrict__ loss) {
+// loss = mean over batch x 6 of (y - t)^2, by block 0 (256 threads, each over its own entries, then a
+// tree: one order whatever the batch); dY = d loss / dy (BF16, the 6 outputs of 16 columns) by the others.
+__global__ void __launch_bounds__(256) mse_kernel(const float* __restrict__ Y, const float* __restrict__ T, int batch,
+                                                  bf16* __restrict__ dY, float* __restrict__ loss) {
   __shared__ float red[256];
-  float s = 0.f;
   const float scale = 2.f / (float)(batch * kOut);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < batch * kOutP; i += gridDim.x * blockDim.x) {
+  if (blockIdx.x > 0) {
+    const int i = (blockIdx.x - 1) * 256 + threadIdx.x, b = i / kOutP, j = i % kOutP;
+    if (i >= batch * kOutP) return;
+    dY[i] = __float2bfloat16_rn(j < kOut ? scale * (Y[i] - T[(size_t)b * kOut + j]) : 0.f);
+    return;
+  }
+  float s = 0.f;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < batch * kOutP; i += 256) {
     const int b = i / kOutP, j = i % kOutP;
-    float g = 0.f;
     if (j < kOut) {
-      const float d = Y[(size_t)b * kOutP + j] - T[(size_t)b * kOut + j];
+      const float d = Y[i] - T[(size_t)b * kOut + j];
       s += d * d;
-      g = scale * d;
     }
-    dY[i] = __float2bfloat16_rn(g);
   }
   red[threadIdx.x] = s;
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+  for (int o = 128; o > 0; o >>= 1) {
     if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) atomicAdd(loss, red[0] / (float)(batch * kOut));
+  if (threadIdx.x == 0) *loss = red[0] / (float)(batch * kOut);
 }
 
-// db[c] += sum over rows of dZ[r, c] (Cn a multiple of 8, at most 128): each block sums a chunk of
-// rows, column by column in row order, with one atomic per column.
+// Column sums of dZ (R x Cn, Cn a multiple of 8, at most 128): each block sums a chunk of rows,
+// column by column in row order, into its row of part; add_parts_kernel adds the rows.
 //
 // The serial sum of a chunk (2 242 rows for conv1) is fixed, so its latency is what can be had: the
 // block brings tiles of rows to shared memory (16-byte loads, the next tile's in flight) and one
@@ -782,12 +787,11 @@ __global__ void mse_kernel(const float* __restrict__ Y, const float* __restrict_
 // training step of 256 took 251 us (139 us for conv1's 331 776 rows), now 55 us.
 constexpr int kBiasThreads = 256, kBiasTile = 16384;  // bytes per tile
 __global__ void __launch_bounds__(kBiasThreads) bias_grad_kernel(const bf16* __restrict__ dZ, long long R, int Cn,
-                                                                 float* __restrict__ db) {
+                                                                 float* __restrict__ part) {
   __shared__ __align__(16) unsigned char tile[kBiasTile];
   constexpr int kPer = kBiasTile / 16 / kBiasThreads;  // 16-byte chunks per thread and tile
   const long long per = (R + gridDim.x - 1) / gridDim.x, r0 = blockIdx.x * per;
   const long long rows = r0 + per < R ? per : R - r0;
-  if (rows <= 0) return;
   const int tid = threadIdx.x, trows = kBiasTile / (2 * Cn);
   const uint4* src = reinterpret_cast<const uint4*>(dZ + r0 * Cn);
   const long long chunks = rows * Cn / 8;
@@ -821,7 +825,51 @@ __global__ void __launch_bounds__(kBiasThreads) bias_grad_kernel(const bf16* __r
       for (; r < m; ++r) s += __bfloat162float(c[r * Cn]);
     }
   }
-  if (tid < Cn) atomicAdd(db + tid, s);
+  if (tid < Cn) part[(size_t)blockIdx.x * Cn + tid] = s;
+}
+
+// Sources of a gradient: `splits` partial sums of the entries first .. first + count - 1 of the flat
+// vector, stride apart.  Two sources of the same entries (conv1 and conv2 on the reference subset and
+// on the deformed window) are added one after the other.
+struct GradSource {
+  const float* part;
+  long long stride;
+  int first, count, splits;
+};
+struct GradSources {
+  GradSource s[16];
+  int n;
+};
+
+// g = the sources' partial sums, every entry's added in one order (source by source, split by split)
+// in FP64 and rounded once.  Atomics in the order of arrival left the last bits to chance, and over
+// Adam steps a flipped BF16 rounding of a weight carries that into all parameters; the order of arrival
+// also shifted with the GEMM's tile width (its waves), by 2e-7 of conv2's gradient.  Bound by the latency
+// of its loads (24 MB of partial sums at batch 256, in L2): 32 of them are in flight.
+__global__ void __launch_bounds__(256) add_parts_kernel(const __grid_constant__ GradSources src, long long n,
+                                                        float* __restrict__ g) {
+  const long long i = blockIdx.x * 256LL + threadIdx.x;
+  if (i >= n) return;
+  double s = 0.0;
+  bool any = false;
+  for (int q = 0; q < src.n; ++q) {
+    const GradSource& c = src.s[q];
+    const long long e = i - c.first;
+    if (e < 0 || e >= c.count) continue;
+    any = true;
+    const float* p = c.part + e;
+    int k = 0;
+    for (; k + 32 <= c.splits; k += 32) {
+      float x[32];
+#pragma unroll
+      for (int u = 0; u < 32; ++u) x[u] = __ldcg(p + (k + u) * c.stride);
+#pragma unroll
+      for (int u = 0; u < 32; ++u) s += x[u];
+    }
+#pragma unroll 8
+    for (; k < c.splits; ++k) s += __ldcg(p + k * c.stride);
+  }
+  if (any) g[i] = (float)s;
 }
 
 // Adam (Kingma & Ba 2015) on the flat FP32 parameters, refreshing their BF16 copies
@@ -917,6 +965,9 @@ struct ProposalNet {
   bool w4d_valid = false;                 // W4d, W4dT, b4d match the current weights
   bf16 *dY = nullptr, *dYt = nullptr;
   float *dAf = nullptr, *dHf = nullptr, *Y = nullptr, *loss = nullptr;
+  float* parts = nullptr;  // partial sums of the weight and bias gradients of one step
+  size_t parts_used = 0;
+  GradSources src{};       // where they lie
   uint8_t* ok = nullptr;  // per predicted subset: its feature crops lie inside the maps
   // whole-image features for prediction (sized for the last frame size): the reference and
   // deformed conv2 maps
@@ -945,7 +996,8 @@ namespace {
 long long P_of(int i, int batch) { return (long long)batch * kConv[i].Hout * kConv[i].Hout; }
 
 int gemm(ProposalNet* net, const void* A, long long lda, const void* B, long long ldb, long long M, long long N,
-         long long K, int mode, float* c32, bf16* c16, const float* bias, long long ldc, int splits) {
+         long long K, int mode, float* c32, bf16* c16, const float* bias, long long ldc, int splits,
+         long long split_stride = 0) {
   GemmArgs ga;
   ga.A = A;
   ga.lda = lda;
@@ -960,6 +1012,7 @@ int gemm(ProposalNet* net, const void* A, long long lda, const void* B, long lon
   ga.epi.c16 = c16;
   ga.epi.bias = bias;
   ga.epi.ldc = ldc;
+  ga.epi.split_stride = split_stride;
   ga.epi.err = net->errflag;
   const int r = launch_umma_gemm(ga, net->stream);
   if (r < 0) {
@@ -976,11 +1029,6 @@ void transpose(ProposalNet* net, const bf16* in, bf16* out, long long R, long lo
   ++net->launches;
 }
 
-void bias_grad(ProposalNet* net, const bf16* dZ, long long R, int Cn, float* db, int blocks = 148) {
-  bias_grad_kernel<<<blocks, kBiasThreads, 0, net->stream>>>(dZ, R, Cn, db);
-  ++net->launches;
-}
-
 // split-K count for a weight gradient: enough blocks to fill the SMs
 int wsplit(long long M, long long N, long long K) {
   const long long tiles = ((M + 127) / 128) * ((N + 255) / 256);
@@ -988,6 +1036,42 @@ int wsplit(long long M, long long N, long long K) {
   const long long kb = (K + 63) / 64;
   if (s > kb) s = kb;
   return (int)(s < 1 ? 1 : s);
+}
+
+constexpr int kBiasBlocks = 148;
+
+// Room for the partial sums of one step at up to `batch` samples (floats).
+size_t parts_floats(long long batch) {
+  size_t n = kFcHid * kOutP * (size_t)wsplit(kOutP, kFcHid, batch) + (size_t)kFcHid * kFcIn * wsplit(kFcHid, kFcIn, batch);
+  for (int i = 0; i < kNumConv; ++i) {
+    const ConvI& L = kConv[i];
+    if (i != kConv4)  // conv4's is one dense product, folded
+      n += (size_t)L.Cout * L.Kp * wsplit(L.Cout, L.Kp, batch * L.Hout * L.Hout);
+    n += (size_t)kBiasBlocks * L.Cout;
+  }
+  return n + (size_t)kBiasBlocks * (kFcHid + kOutP);
+}
+
+// The next source of the step's gradients: partial sums of the entries from `first` on.
+float* take_parts(ProposalNet* net, long long first, long long count, int splits) {
+  float* p = net->parts + net->parts_used;
+  net->src.s[net->src.n++] = GradSource{p, count, (int)first, (int)count, splits};
+  net->parts_used += (size_t)count * splits;
+  return p;
+}
+
+// Partial bias gradients: the column sums of dZ (R x Cn).
+void bias_grad(ProposalNet* net, const bf16* dZ, long long R, int Cn, long long first, int blocks = kBiasBlocks) {
+  bias_grad_kernel<<<blocks, kBiasThreads, 0, net->stream>>>(dZ, R, Cn, take_parts(net, first, Cn, blocks));
+  ++net->launches;
+}
+
+// Partial weight gradients dW (M x N) = At Bt^T over K samples, one per K range.
+int weight_grad(ProposalNet* net, const bf16* At, const bf16* Bt, long long M, long long N, long long K,
+                long long first) {
+  const int splits = gemm_splits(K, wsplit(M, N, K));
+  return gemm(net, At, K, Bt, K, M, N, K, kEpiStore, take_parts(net, first, M * N, splits), nullptr, nullptr, N, splits,
+              M * N);
 }
 
 // im2col rows of convolution i's input (at `in` seen through v) into net->A[i]
@@ -1065,16 +1149,15 @@ int forward(ProposalNet* net, int batch, const bf16* X) {
   return rc ? rc : head(net, batch);
 }
 
-// weight and bias gradients of convolution i from its output gradient dZ[i] (added to net->g)
+// weight and bias gradients of convolution i from its output gradient dZ[i] (partial sums)
 int conv_wgrad(ProposalNet* net, int i, int batch) {
   const ConvI& L = kConv[i];
   const long long P = P_of(i, batch);
   transpose(net, net->dZ[i], net->dZt[i], P, L.Cout);
   transpose(net, net->A[i], net->At[i], P, L.Kp);
-  int rc = gemm(net, net->dZt[i], P, net->At[i], P, L.Cout, L.Kp, P, kEpiAtomic, net->g + kL.w[L.layer], nullptr,
-                nullptr, L.Kp, wsplit(L.Cout, L.Kp, P));
+  int rc = weight_grad(net, net->dZt[i], net->At[i], L.Cout, L.Kp, P, kL.w[L.layer]);
   if (rc) return rc;
-  bias_grad(net, net->dZ[i], P, L.Cout, net->g + kL.b[L.layer]);
+  bias_grad(net, net->dZ[i], P, L.Cout, kL.b[L.layer]);
   return ALDIC_OK;
 }
 
@@ -1100,33 +1183,31 @@ void relu_grad(ProposalNet* net, const bf16* H, bf16* dZ, long long n) {
   ++net->launches;
 }
 
-// gradients of the mean squared error into net->g (zeroed here)
+// gradients of the mean squared error into net->g
 int backward(ProposalNet* net, int batch, const bf16* X, const float* T) {
   cudaStream_t st = net->stream;
   const long long B = batch;
-  NK(cudaMemsetAsync(net->g, 0, sizeof(float) * kL.n, st));
-  NK(cudaMemsetAsync(net->loss, 0, sizeof(float), st));
-  mse_kernel<<<(unsigned)((batch * kOutP + 255) / 256), 256, 0, st>>>(net->Y, T, batch, net->dY, net->loss);
+  net->src.n = 0;
+  net->parts_used = 0;
+  mse_kernel<<<1 + (unsigned)((batch * kOutP + 255) / 256), 256, 0, st>>>(net->Y, T, batch, net->dY, net->loss);
   ++net->launches;
   // transposed weights for the data gradients (conv1's input needs none)
   for (int l = 1; l < 6; ++l) transpose(net, net->wb + kL.w[l], net->wt[l], kL.rows[l], kL.cols[l]);
   // FC2: dW = dY^T H6, db = sum dY, dH6 = dY W
   transpose(net, net->dY, net->dYt, B, kOutP);
   transpose(net, net->H6, net->Ht6, B, kFcHid);
-  int rc = gemm(net, net->dYt, B, net->Ht6, B, kOutP, kFcHid, B, kEpiAtomic, net->g + kL.w[5], nullptr, nullptr,
-                kFcHid, wsplit(kOutP, kFcHid, B));
+  int rc = weight_grad(net, net->dYt, net->Ht6, kOutP, kFcHid, B, kL.w[5]);
   if (rc) return rc;
-  bias_grad(net, net->dY, B, kOutP, net->g + kL.b[5], 64);
+  bias_grad(net, net->dY, B, kOutP, kL.b[5], 64);
   rc = gemm(net, net->dY, kOutP, net->wt[5], kOutP, B, kFcHid, kOutP, kEpiStore, net->dHf, nullptr, nullptr, kFcHid, 1);
   if (rc) return rc;
   relu_grad(net, net->H6, net->dZ6, B * kFcHid);
   // FC1: dW = dZ6^T F, db, dF = dZ6 W (F = conv4's output, flattened)
   transpose(net, net->dZ6, net->dZt6, B, kFcHid);
   transpose(net, net->H[kConv4], net->Ht5, B, kFcIn);
-  rc = gemm(net, net->dZt6, B, net->Ht5, B, kFcHid, kFcIn, B, kEpiAtomic, net->g + kL.w[4], nullptr, nullptr, kFcIn,
-            wsplit(kFcHid, kFcIn, B));
+  rc = weight_grad(net, net->dZt6, net->Ht5, kFcHid, kFcIn, B, kL.w[4]);
   if (rc) return rc;
-  bias_grad(net, net->dZ6, B, kFcHid, net->g + kL.b[4], 64);
+  bias_grad(net, net->dZ6, B, kFcHid, kL.b[4], 64);
   rc = gemm(net, net->dZ6, kFcHid, net->wt[4], kFcHid, B, kFcIn, kFcHid, kEpiStore, net->dHf, nullptr, nullptr, kFcIn,
             1);
   if (rc) return rc;
@@ -1140,7 +1221,7 @@ int backward(ProposalNet* net, int batch, const bf16* X, const float* T) {
   if (rc) return rc;
   conv4_fold_kernel<<<144, 256, 0, st>>>(net->dAf, net->g + kL.w[3]);
   ++net->launches;
-  bias_grad(net, net->dZ[kConv4], B * 16, 64, net->g + kL.b[3]);
+  bias_grad(net, net->dZ[kConv4], B * 16, 64, kL.b[3]);
   rc = gemm(net, net->dZ[kConv4], kFcIn, net->W4dT, kFcIn, B, kFcIn, kFcIn, kEpiStore, net->dHf, nullptr, nullptr,
             kFcIn, 1);
   if (rc) return rc;
@@ -1161,7 +1242,10 @@ int backward(ProposalNet* net, int batch, const bf16* X, const float* T) {
       (rc = conv_dgrad(net, kConvD2, batch, net->H[kConvD1], net->dZ[kConvD1])))
     return rc;
   im2col(net, kConvD1, batch, X, kViewDef);
-  return conv_wgrad(net, kConvD1, batch);
+  if ((rc = conv_wgrad(net, kConvD1, batch))) return rc;
+  add_parts_kernel<<<(unsigned)((kL.n + 255) / 256), 256, 0, st>>>(net->src, kL.n, net->g);
+  ++net->launches;
+  return ALDIC_OK;
 }
 
 int check_errflag(ProposalNet* net) {
@@ -1238,6 +1322,7 @@ int aldic_net_create(aldic_net** out, int device, int max_batch) {
   if (e == cudaSuccess) e = cudaMalloc(&net->dAf, maxA * 4);
   if (e == cudaSuccess) e = cudaMalloc(&net->dHf, maxH * 4);
   if (e == cudaSuccess) e = cudaMalloc(&net->loss, 4);
+  if (e == cudaSuccess) e = cudaMalloc(&net->parts, parts_floats(B) * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&net->ok, B);
   if (e == cudaSuccess) e = cudaMalloc(&net->errflag, 4);
   if (e != cudaSuccess) return fail(e);
@@ -1256,7 +1341,7 @@ void aldic_net_destroy(aldic_net* net) {
   if (net->stream) cudaStreamSynchronize(net->stream);
   void* bufs[] = {net->w,  net->g,   net->m,   net->v,   net->wb,  net->Ht5, net->H6,     net->Ht6,
                   net->dZ6, net->dZt6, net->dY, net->dYt, net->Y, net->dAf, net->dHf, net->loss, net->ok,  net->errflag,
-                  net->FR, net->FD, net->W4d, net->W4dT, net->b4d};
+                  net->FR, net->FD, net->W4d, net->W4dT, net->b4d, net->parts};
   for (void* p : bufs)
     if (p) cudaFree(p);
   for (int l = 0; l < 6; ++l)

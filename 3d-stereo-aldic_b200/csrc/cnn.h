@@ -6,8 +6,8 @@
 
 namespace aldic {
 
-constexpr int kEpiStore = 0;         // c32[r, c] = acc (+ bias[c])
-constexpr int kEpiAtomic = 1;        // c32[r, c] += acc (split-K partial sums)
+constexpr int kEpiStore = 0;         // c32[r, c] = acc (+ bias[c]); with splits, split k's at c32 + k split_stride
+constexpr int kEpiAtomic = 1;        // c32[r, c] += acc (split-K partial sums, in no fixed order)
 constexpr int kEpiBiasReluBf16 = 2;  // c16[r, c] = bf16(max(acc + bias[c], 0))
 
 struct GemmEpi {
@@ -16,13 +16,14 @@ struct GemmEpi {
   __nv_bfloat16* c16;
   const float* bias;  // N entries or null
   long long ldc;      // row pitch of the output (elements)
+  long long split_stride = 0;  // kEpiStore: elements between the outputs of two splits
   int* err;           // set (bit 0: a load or MMA wait timed out; bit 1: the epilogue's) on failure
 };
 
 // C[M x N] = A[M x K] * B[N x K]^T; A and B row-major BF16 with row pitches lda / ldb
 // (elements, multiples of 8 so rows start on 16-byte boundaries), 16-byte aligned bases.
 // Rows of A or B beyond M / N and columns beyond K read as zero.  splits > 1 divides K over
-// that many blocks per tile (epilogue kEpiAtomic only).
+// that many blocks per tile (kEpiAtomic, or kEpiStore with a split_stride).
 struct GemmArgs {
   const void* A;
   long long lda;
@@ -34,5 +35,7 @@ struct GemmArgs {
 };
 
 int launch_umma_gemm(const GemmArgs& g, cudaStream_t st);
+// The K ranges that a GEMM asked for `splits` of them runs (each holds at least one K block).
+int gemm_splits(long long K, int splits);
 
 }  // namespace aldic

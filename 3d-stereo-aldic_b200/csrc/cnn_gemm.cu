@@ -71,7 +71,7 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmEpi& epi, uint32_t 
     // bytes a lane and a row a lane apart, the stores of conv2's data gradient took 82 us; so
     // 27 us, in tiles of 96 columns)
     const int lane = threadIdx.x & 31, row0 = row - lane;
-    if (epi.mode == kEpiStore && epi.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(epi.c32) & 15) == 0) {
+    if (stage && epi.mode == kEpiStore && epi.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(epi.c32) & 15) == 0) {
 #pragma unroll 1
       for (; c_first < BN && n0 + c_first + 32 <= N; c_first += 32) {
         float v[32];
@@ -167,7 +167,7 @@ __device__ __forceinline__ void gemm_epilogue_tile(const GemmEpi& epi, uint32_t 
 template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     umma_gemm_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, GemmEpi epi,
-                     int M, int N, TileGrid tg) {
+                     int M, int N, TileGrid tg, int staged) {
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "UMMA N");
   constexpr uint32_t kCols = GemmSmem<BN>::acc_cols;
   constexpr uint32_t kAlloc = 2 * kCols;  // two accumulators (a power of two, <= 512)
@@ -275,9 +275,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         break;
       }
       tcgen05_after_sync();
-      gemm_epilogue_tile<BN>(epi, tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)b * kCols, m0 + q * 32 + lane,
+      GemmEpi out = epi;
+      out.c32 += kb0 / tg.kb_per_split * epi.split_stride;
+      gemm_epilogue_tile<BN>(out, tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)b * kCols, m0 + q * 32 + lane,
                              nt * BN, M, N,
-                             reinterpret_cast<float*>(smem + kStages * GemmSmem<BN>::stage_bytes) + q * 32 * 36);
+                             staged ? reinterpret_cast<float*>(smem + kStages * GemmSmem<BN>::stage_bytes) + q * 32 * 36
+                                    : nullptr);
       tcgen05_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[b]);
@@ -329,6 +332,18 @@ int num_sms() {
   return sms;
 }
 
+}  // namespace
+
+int gemm_splits(long long K, int splits) {
+  const int kb = (int)((K + kBK - 1) / kBK);
+  if (splits < 1) splits = 1;
+  if (splits > kb) splits = kb;
+  const int per = (kb + splits - 1) / splits;
+  return (kb + per - 1) / per;
+}
+
+namespace {
+
 template <int BN>
 int launch_bn(const GemmArgs& g, cudaStream_t st) {
   CUtensorMap ta, tb;
@@ -336,11 +351,8 @@ int launch_bn(const GemmArgs& g, cudaStream_t st) {
   std::memset(&tb, 0, sizeof(tb));
   if (!make_tmap_bf16(&ta, g.A, g.M, g.K, g.lda, 128) || !make_tmap_bf16(&tb, g.B, g.N, g.K, g.ldb, BN)) return -1;
   const int kb_total = (int)((g.K + kBK - 1) / kBK);
-  int splits = g.splits < 1 ? 1 : g.splits;
-  if (splits > kb_total) splits = kb_total;
-  const int per = (kb_total + splits - 1) / splits;
-  splits = (kb_total + per - 1) / per;  // every split holds at least one K block
-  if (splits > 1 && g.epi.mode != kEpiAtomic) return -1;
+  const int splits = gemm_splits(g.K, g.splits), per = (kb_total + splits - 1) / splits;
+  if (splits > 1 && g.epi.mode != kEpiAtomic && !(g.epi.mode == kEpiStore && g.epi.split_stride > 0)) return -1;
   TileGrid tg;
   tg.tiles_m = (int)((g.M + 127) / 128);
   tg.tiles_n = (int)((g.N + BN - 1) / BN);
@@ -349,14 +361,17 @@ int launch_bn(const GemmArgs& g, cudaStream_t st) {
   tg.kb_total = kb_total;
   // persistent: as many CTAs as fit on the GPU at once (shared memory bound), at most one
   // per tile
-  const int bytes = GemmSmem<BN>::bytes + (g.epi.mode == kEpiStore ? GemmSmem<BN>::store_bytes : 0);
+  // per tile; the partial tiles of splits are few and narrow, and gain more from a second CTA an SM
+  // than from staged stores
+  const int staged = g.epi.mode == kEpiStore && BN % 32 == 0 && splits == 1;
+  const int bytes = GemmSmem<BN>::bytes + (staged ? GemmSmem<BN>::store_bytes : 0);
   const long long slots = (long long)num_sms() * std::min(4, (227 * 1024) / bytes);
   const int grid = (int)(tg.ntiles < slots ? tg.ntiles : slots);
   auto k = umma_gemm_kernel<BN>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        GemmSmem<BN>::bytes + GemmSmem<BN>::store_bytes);
   cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  k<<<grid, kGemmThreads, bytes, st>>>(ta, tb, g.epi, (int)g.M, (int)g.N, tg);
+  k<<<grid, kGemmThreads, bytes, st>>>(ta, tb, g.epi, (int)g.M, (int)g.N, tg, staged);
   return 1;
 }
 
