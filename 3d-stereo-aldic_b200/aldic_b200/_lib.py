@@ -20,7 +20,7 @@ SLOT_REF, SLOT_DEF = 0, 1
 UNIFORM, QUADTREE = 0, 1
 OPT_ITERATION_CAP, OPT_STAGING, OPT_SLOW_WARPS, OPT_SEARCH_IMPL, OPT_SEARCH_CHUNK, OPT_AUTOTUNE = 0, 1, 2, 3, 4, 5
 OPT_SLOW_FP64, OPT_FP64_THREADS = 6, 7
-STAT_FP64_RESOLVES, STAT_STAGING_TIMEOUT = 100, 101
+STAT_FP64_RESOLVES, STAT_STAGING_TIMEOUT, STAT_SEARCH_LEFT = 100, 101, 102
 # iterations the one-warp solver pass gives a subset before the multi-warp pass restarts it, when
 # aldic_set_iteration_cap has not been called (kDefaultWarpCap in csrc/kernels.h)
 DEFAULT_ITERATION_CAP = 8

@@ -27,6 +27,8 @@ struct Arena {
   size_t cap = 0, used = 0;
 };
 
+constexpr int kSearchLeft = 16;  // entry of aldic_ctx::qcount that no other call clears
+
 }  // namespace
 
 struct aldic_ctx {
@@ -50,7 +52,7 @@ struct aldic_ctx {
   double* partials = nullptr;
   unsigned int* counter = nullptr;
   int npartials = 0;
-  int* qcount = nullptr;
+  int* qcount = nullptr;  // 32 ints: IC-GN's and Subpb1's queue counters, then kSearchLeft
   int* sel_count = nullptr;  // aldic_fallback_select's counter
   double* I1 = nullptr;
   double* I2 = nullptr;
@@ -67,6 +69,7 @@ struct aldic_ctx {
   int slow_nw = 2;      // ALDIC_OPT_SLOW_WARPS (FP32 slow pass, with ALDIC_OPT_SLOW_FP64 0)
   int slow_fp64 = 0;    // ALDIC_OPT_SLOW_FP64
   int fp64_threads = 128;  // ALDIC_OPT_FP64_THREADS
+  int search_path = kSearchDirect;  // the kernel of the last search
   int search_impl = 0;  // ALDIC_OPT_SEARCH_IMPL
   int search_chunk = 0; // ALDIC_OPT_SEARCH_CHUNK
   int autotune = 0;     // ALDIC_OPT_AUTOTUNE
@@ -262,7 +265,7 @@ int aldic_create(aldic_ctx** out, int device) {
     if (e == cudaSuccess) e = cudaMalloc(&c->partials, c->npartials * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&c->counter, 64);
     if (e == cudaSuccess) e = cudaMemset(c->counter, 0, 64);
-    if (e == cudaSuccess) e = cudaMalloc(&c->qcount, 64);
+    if (e == cudaSuccess) e = cudaMalloc(&c->qcount, 128);
   }
   if (e != cudaSuccess) {
     delete c;
@@ -543,6 +546,8 @@ static int search_common(aldic_ctx* c, const int* search, const int* gridx, cons
   a.tot = c->iitot;
   a.tile_scratch = tbytes ? c->tscratch : nullptr;
   a.ev_start = a.ev_stop = nullptr;
+  a.left = c->qcount + kSearchLeft;
+  a.path = &c->search_path;
   a.impl = c->search_impl;
   a.chunk = c->search_chunk;
   a.list = (const int*)al.dev;
@@ -1521,6 +1526,13 @@ int aldic_get_option(aldic_ctx* c, int option, int* value) {
       *value = option == ALDIC_STAT_FP64_RESOLVES ? q[4] : q[8];
       return ALDIC_OK;
     }
+    case ALDIC_STAT_SEARCH_LEFT:
+      *value = 0;
+      if (c->search_path != kSearchFft) return ALDIC_OK;
+      CK(cudaSetDevice(c->device));
+      CK(cudaMemcpyAsync(value, c->qcount + kSearchLeft, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      return ALDIC_OK;
     default:
       return fail(c, ALDIC_ERR_ARG, "unknown option %d", option);
   }

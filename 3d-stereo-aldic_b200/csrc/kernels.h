@@ -103,7 +103,10 @@ struct SearchArgs {
   long long nlist;
   const int* dlist = nullptr;   // direct kernel: the subsets to search (outputs in the grid's slots) and
   const int* dcount = nullptr;  // their number, both on the device; null for the whole grid
+  int* left = nullptr;   // device: receives the number of subsets that the transforms leave to direct sums
+  int* path = nullptr;   // host, or null: the kernel that launch_search took, kSearchFft and so on
 };
+constexpr int kSearchFft = 0, kSearchTile = 1, kSearchDirect = 2;
 // Whether a shared-product tile kernel exists for (step, w + 1) and fits this device.
 bool search_tile_available(int step, int winsize, int chunk);
 

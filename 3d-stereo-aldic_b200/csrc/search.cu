@@ -462,10 +462,14 @@ int launch_search(const SearchArgs& a, cudaStream_t st) {
   launch_integral(a.g, a.M, a.N, a.I1, a.I2, a.tot, st);
   // transforms, or shared products over tiles of subsets where a tile kernel exists for (step, w + 1)
   // (a subset list takes the direct kernel)
+  int path, &took = a.path ? *a.path : path;
+  took = kSearchFft;
   const int fl = launch_search_fft(a, st);
   if (fl >= 0) return 3 + fl;
+  took = kSearchTile;
   const int tl = a.list ? -1 : launch_search_tile(a, st);
   if (tl >= 0) return 3 + tl;
+  took = kSearchDirect;
   const int l = launch_search_direct(a, st);
   return l < 0 ? l : 3 + l;
 }

@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(FftShape<L>::NT, FftShape<L>::MINB)
     for (int it = tid; it < NPO * 16; it += NT) {
       const int n1 = it & 15, p = it >> 4;
       // 1 / sqrt of the variance sums of both rows' shifts (NaN outside the crop, which no maximum
-      // takes; 0 for a window of zeros), fetched ahead of the transform.  Where the sum is near the
+      // takes; 0 for a flat window), fetched ahead of the transform.  Where the sum is near the
       // zero threshold the bounds lie so far apart that the shift is a candidate.
       float rs[2][B];
 #pragma unroll
@@ -565,7 +565,7 @@ int launch_fft(const SearchArgs& a, const SearchTables& t, cudaStream_t st) {
     fft_rows_kernel<L><<<dim3((a.M + 2 * kRowPairs - 1) / (2 * kRowPairs), nj), kRowThreads, rsmem, st>>>(a, jb, (float2*)t.rows);
     const unsigned grid = (unsigned)std::min<long long>((long long)a.nx * nj, (long long)sms * per);
     kern<<<grid, FftShape<L>::NT, smem, st>>>(a, jb, nj, (const float2*)t.rows, t.map, t.prm, t.ringv,
-                                                 t.best, t.flist + 1, t.flist);
+                                                 t.best, t.flist, a.left);
     launches += 2;
   }
   return launches;
@@ -619,7 +619,7 @@ int launch_search_fft(const SearchArgs& a, cudaStream_t st) {
   if (!L) return -1;
   SearchTables t;
   const int launches = launch_search_tables(a, row_bytes(L, a.M) * row_columns(L, a.M, a.ny), &t, st);
-  if (cudaMemsetAsync(t.flist, 0, sizeof(int), st) != cudaSuccess) return -1;
+  if (cudaMemsetAsync(a.left, 0, sizeof(int), st) != cudaSuccess) return -1;
   if (a.ev_start) cudaEventRecord(a.ev_start, st);
   int l = -1;
   switch (L) {
@@ -635,8 +635,8 @@ int launch_search_fft(const SearchArgs& a, cudaStream_t st) {
   if (l < 0) return -1;
   SearchArgs d = a;  // the subsets left to direct sums
   d.ev_start = d.ev_stop = nullptr;
-  d.dlist = t.flist + 1;
-  d.dcount = t.flist;
+  d.dlist = t.flist;
+  d.dcount = a.left;
   const int ld = launch_search_direct(d, st);
   if (ld < 0) return -1;
   if (a.ev_stop) cudaEventRecord(a.ev_stop, st);

@@ -7,11 +7,11 @@
 namespace aldic {
 
 struct SearchTables {
-  const float* map;      // 1 / sqrt of the variance sum of every full window position, row-major; 0: a window of zeros
+  const float* map;      // 1 / sqrt of the variance sum of every full window position, row-major; 0: a flat window
   const SubsetPrm* prm;  // per subset
   const float2* ringv;   // per subset: (mean, 1 / sqrt) of the partial windows
   int* best;             // per subset: crop index of the first maximum, -1 where the direct kernel decides
-  int* flist;            // a count, then those subsets
+  int* flist;            // those subsets (their number: SearchArgs::left)
   void* rows;            // row spectra
 };
 

@@ -93,7 +93,7 @@ struct TileScratch {
   double* vb;        // MW x ceil(NW / kVB): largest V of every kVB consecutive columns
   double* rr;        // nx x 2 sides x 4 x (N+1): integral-image rows of the top / bottom ring windows
   void* rows;        // row spectra of the transforms
-  int* flist;        // nx * ny + 1: a count, then the subsets that the transforms leave to direct sums
+  int* flist;        // nx * ny: the subsets that the transforms leave to direct sums
 };
 
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -117,7 +117,7 @@ inline size_t scratch_layout(int M, int N, int W1, int nx, int ny, int nda, size
   char* pf = take(n * sizeof(float));  // >= the number of tiles
   char* prr = take((size_t)nx * 8 * (size_t)(N + 1) * sizeof(double));
   char* pvb = take(MW * ((NW + kVB - 1) / kVB) * sizeof(double));
-  char* pl = take((n + 1) * sizeof(int));
+  char* pl = take(n * sizeof(int));
   char* pw = take(row_bytes);
   if (sc) {
     sc->flist = (int*)pl;
@@ -138,9 +138,15 @@ inline size_t scratch_layout(int M, int N, int W1, int nx, int ny, int nda, size
 
 __device__ __forceinline__ float rsqrt_from(double v) { return v > 0 ? (float)(1.0 / sqrt(v)) : INFINITY; }
 
-// Whether a window's sum of squares is no more than the rounding of the integral image (its corner):
-// a window of zeros, as under a mask.  Its products are exactly zero, which a transform does not give.
-__device__ __forceinline__ bool is_zero(double S2, double corner) { return S2 <= 3.6e-15 * corner; }
+// Whether a window's variance sum is no more than the rounding of the integral images (corner: the
+// prefix sum of g^2 at the window's last pixel): a window of one value, as under a mask or where the
+// camera is saturated.  Its normalised values are rounding over rounding; they count as 0.  A
+// transform's error over such a variance would make every shift there a possible maximum, and 33 of
+// them send the subset to direct sums (on 2048 x 2048 with a constant band and disc, window 41 at radius
+// 70: 14.0 ms so, 7.2 ms with this test).  Windows of one value come out at up to 45 times 2^-52
+// corner (the tiles' sums restated in numpy: 333 x 401 to 4096 x 3000, windows 21 to 61); 128 leaves a
+// margin of three, and a variance below it has no digit to trust.
+__device__ __forceinline__ bool is_flat(double v, double corner) { return v <= 128 * 2.2204460492503131e-16 * corner; }
 
 }  // namespace
 
@@ -169,7 +175,7 @@ __global__ void __launch_bounds__(256) window_map_kernel(const double* __restric
       box_sums(x, x + W1 - 1, y, y + W1 - 1, I1, I2, (size_t)M + 1, &S1, &S2);
       v = S2 - S1 * S1 / nwin;
       if constexpr (sizeof(T) == sizeof(float))
-        m = v <= 0 || is_zero(S2, I2[(size_t)(x + W1) + (size_t)(y + W1) * ((size_t)M + 1)]) ? 0.f : rsqrt_from(v);
+        m = v <= 0 || is_flat(v, I2[(size_t)(x + W1) + (size_t)(y + W1) * ((size_t)M + 1)]) ? 0.f : rsqrt_from(v);
       else
         m = make_float2((float)(S1 / nwin), rsqrt_from(v));
     }
@@ -241,7 +247,7 @@ __global__ void ring_rows_kernel(SearchArgs a, double* __restrict__ rr) {
 }
 
 // One warp per subset: template mean and norm, the window sums of the ring of partial
-// windows (zeros: 0 for the 1 / sqrt of a window of zeros), the largest window variance sum over the
+// windows (zeros: 0 for the 1 / sqrt of a flat window), the largest window variance sum over the
 // crop (normxcorr2 zero threshold) and validity; writes x, y and the NaN outputs of invalid subsets.
 //
 // Bound by the latency of its loads: the template's offsets are stepped (a division per sample took
@@ -317,7 +323,7 @@ __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const
           const double S2 = (R[3 * N1 + c1 + 1] - R[3 * N1 + c0]) - (R[2 * N1 + c1 + 1] - R[2 * N1 + c0]);
           const double v = S2 - S1 * S1 / nwin;
           m = fmax(m, v);
-          rv[side * nda + bb] = make_float2((float)(S1 / nwin), zeros && (v <= 0 || is_zero(S2, R[3 * N1 + c1 + 1])) ? 0.f : rsqrt_from(v));
+          rv[side * nda + bb] = make_float2((float)(S1 / nwin), zeros && (v <= 0 || is_flat(v, R[3 * N1 + c1 + 1])) ? 0.f : rsqrt_from(v));
         }
       }
       for (int k = lane; k < 2 * s.na; k += 32) {
@@ -327,7 +333,7 @@ __global__ void __launch_bounds__(256, 4) subset_prep_kernel(SearchArgs a, const
         const double v = S2 - S1 * S1 / nwin;
         m = fmax(m, v);
         const size_t corner = (size_t)(min(s.dr1, s.dr0 - 1 + aa + w) + 1) + (size_t)(min(s.dc1, s.dc0 - 1 + (side ? s.nb - 1 : 0) + w) + 1) * ld;
-        rv[(2 + side) * nda + aa] = make_float2((float)(S1 / nwin), zeros && (v <= 0 || is_zero(S2, a.I2[corner])) ? 0.f : rsqrt_from(v));
+        rv[(2 + side) * nda + aa] = make_float2((float)(S1 / nwin), zeros && (v <= 0 || is_flat(v, a.I2[corner])) ? 0.f : rsqrt_from(v));
       }
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));

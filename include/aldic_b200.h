@@ -386,6 +386,10 @@ int aldic_measure_fp32_peak(aldic_ctx* ctx, double* tflops);
  * on a barrier). */
 #define ALDIC_STAT_FP64_RESOLVES 100
 #define ALDIC_STAT_STAGING_TIMEOUT 101
+/* Read-only, of the last aldic_integer_search or aldic_integer_search_list (waits for it): the
+ * subsets that the correlation by FFTs left to direct sums, because several shifts were too close
+ * to call or values were not finite; 0 where another kernel ran. */
+#define ALDIC_STAT_SEARCH_LEFT 102
 int aldic_set_option(aldic_ctx* ctx, int option, int value);
 int aldic_get_option(aldic_ctx* ctx, int option, int* value);
 /* The autotuner's choices so far as a JSON object {shape key: {"choice": {...}, "ms":
