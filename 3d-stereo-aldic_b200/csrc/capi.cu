@@ -54,11 +54,9 @@ struct aldic_ctx {
   int npartials = 0;
   int* qcount = nullptr;  // 32 ints: IC-GN's and Subpb1's queue counters, then kSearchLeft
   int* sel_count = nullptr;  // aldic_fallback_select's counter
-  double* I1 = nullptr;
-  double* I2 = nullptr;
-  double* iitot = nullptr;
-  size_t ii_cap = 0, iitot_cap = 0;
-  void* tscratch = nullptr;  // shared-product search scratch
+  char* ii = nullptr;  // the search's integral images and their scratch
+  size_t ii_cap = 0;
+  void* tscratch = nullptr;  // scratch of the search by transforms or tiles
   size_t tscratch_cap = 0;
   int warp_cap = kDefaultWarpCap;  // aldic_set_iteration_cap
   double fp64_band = kDefaultFp64Band;  // aldic_set_fp64_band
@@ -280,7 +278,7 @@ void aldic_destroy(aldic_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* bufs[] = {c->img[0], c->img[1], c->mask, c->gx, c->gy, c->stats, c->partials, c->counter, c->qcount,
-                  c->I1, c->I2, c->iitot, c->tscratch, c->arena.base, c->sp2, c->sel_count};
+                  c->ii, c->tscratch, c->arena.base, c->sp2, c->sel_count};
   for (void* b : bufs)
     if (b) cudaFree(b);
   for (cudaEvent_t e : c->prof_ev) cudaEventDestroy(e);
@@ -443,6 +441,7 @@ int aldic_search_grid(const int* gridx, const int* gridy, int winsize, int step,
 }
 
 static int tune_search(aldic_ctx* c, SearchArgs& a);  // the autotuner (below)
+static size_t tune_search_bytes(aldic_ctx* c, SearchArgs a);
 static int search_common(aldic_ctx* c, const int* search, const int* gridx, const int* gridy, int winsize, int step,
                          int64_t nlist, const int32_t* list, double* x, double* y, double* u, double* v, double* phi);
 
@@ -457,6 +456,18 @@ int aldic_integer_search_list(aldic_ctx* c, const int* search, const int* gridx,
   if (!c) return ALDIC_ERR_ARG;
   if (n < 0 || (n > 0 && !list)) return fail(c, ALDIC_ERR_ARG, "a list of n >= 0 grid subsets is required");
   return search_common(c, search, gridx, gridy, winsize, step, n, list, x, y, u, v, phi);
+}
+
+// A buffer of at least `bytes`: kept, or freed and allocated anew (nothing is held after a failure).
+static int grow(aldic_ctx* c, void** p, size_t* cap, size_t bytes) {
+  if (*cap >= bytes) return ALDIC_OK;
+  CK(cudaStreamSynchronize(c->stream));
+  if (*p) CK(cudaFree(*p));
+  *p = nullptr;
+  *cap = 0;
+  CK(cudaMalloc(p, bytes));
+  *cap = bytes;
+  return ALDIC_OK;
 }
 
 static int search_common(aldic_ctx* c, const int* search, const int* gridx, const int* gridy, int winsize, int step,
@@ -475,36 +486,42 @@ static int search_common(aldic_ctx* c, const int* search, const int* gridx, cons
   const size_t n = nlist >= 0 ? (size_t)nlist : ngrid;  // output slots
   if (n == 0 || ngrid == 0) return ALDIC_OK;
   if (!x || !y || !u || !v || !phi) return fail(c, ALDIC_ERR_ARG, "output arrays required");
-  const size_t iin = (size_t)(c->M + 1) * (c->N + 1);
-  if (c->ii_cap < iin) {
-    CK(cudaStreamSynchronize(c->stream));
-    if (c->I1) CK(cudaFree(c->I1));
-    if (c->I2) CK(cudaFree(c->I2));
-    c->I1 = c->I2 = nullptr;
-    c->ii_cap = 0;
-    CK(cudaMalloc(&c->I1, iin * sizeof(double)));
-    CK(cudaMalloc(&c->I2, iin * sizeof(double)));
-    c->ii_cap = iin;
-  }
-  const size_t itot = search_tot_bytes(c->M, c->N);  // depends on the shape, not on the area alone
-  if (c->iitot_cap < itot) {
-    CK(cudaStreamSynchronize(c->stream));
-    if (c->iitot) CK(cudaFree(c->iitot));
-    c->iitot = nullptr;
-    c->iitot_cap = 0;
-    CK(cudaMalloc(&c->iitot, itot));
-    c->iitot_cap = itot;
-  }
-  // scratch for the transforms or the tile kernel wherever the size allows one of them
-  const size_t tbytes = list ? 0 : search_scratch_bytes(c->M, c->N, winsize, step, nx, ny, search[0], search[1]);
-  if (tbytes > c->tscratch_cap) {
-    CK(cudaStreamSynchronize(c->stream));
-    if (c->tscratch) CK(cudaFree(c->tscratch));
-    c->tscratch = nullptr;
-    c->tscratch_cap = 0;
-    CK(cudaMalloc(&c->tscratch, tbytes));
-    c->tscratch_cap = tbytes;
-  }
+  SearchArgs a;
+  a.f = c->img[0];
+  a.g = c->img[1];
+  a.M = c->M;
+  a.N = c->N;
+  a.s0 = search[0];
+  a.s1 = search[1];
+  a.gx0 = gridx[0];
+  a.gx1 = gridx[1];
+  a.gy0 = gridy[0];
+  a.gy1 = gridy[1];
+  a.winsize = winsize;
+  a.step = step;
+  a.nx = nx;
+  a.ny = ny;
+  a.ev_start = a.ev_stop = nullptr;
+  a.left = c->qcount + kSearchLeft;
+  a.path = &c->search_path;
+  a.impl = c->search_impl;
+  a.chunk = c->search_chunk;
+  a.list = list;  // its place on the device below
+  a.nlist = list ? (long long)n : 0;
+  // one block for both integral images and their tile sums
+  const size_t iin = ((size_t)(c->M + 1) * (c->N + 1) * sizeof(double) + 255) & ~size_t(255);
+  rc = grow(c, (void**)&c->ii, &c->ii_cap, 2 * iin + search_tot_bytes(c->M, c->N));
+  if (rc) return rc;
+  a.I1 = (double*)c->ii;
+  a.I2 = (double*)(c->ii + iin);
+  a.tot = (double*)(c->ii + 2 * iin);
+  // the scratch of the kernel that the call takes (a tuning call: of every candidate); the direct kernel,
+  // which needs none, runs where there is no memory for it
+  const bool tune = c->autotune && !list;
+  const size_t want = tune ? tune_search_bytes(c, a) : search_choose(a);
+  if (want > 0 && grow(c, &c->tscratch, &c->tscratch_cap, want) != ALDIC_OK) cudaGetLastError();
+  a.scratch = c->tscratch;
+  a.scratch_bytes = c->tscratch_cap;
   Arg ox{x, n * 8, true, nullptr}, oy{y, n * 8, true, nullptr}, ou{u, n * 8, true, nullptr};
   Arg ov{v, n * 8, true, nullptr}, op{phi, n * 8, true, nullptr};
   Arg al{list, list ? n * 4 : 0, false, nullptr};
@@ -521,38 +538,13 @@ static int search_common(aldic_ctx* c, const int* search, const int* gridx, cons
     for (int32_t t : hl)
       if (t < 0 || (size_t)t >= ngrid) return fail(c, ALDIC_ERR_ARG, "list entry %d outside the grid of %zu", (int)t, ngrid);
   }
-  SearchArgs a;
-  a.f = c->img[0];
-  a.g = c->img[1];
-  a.M = c->M;
-  a.N = c->N;
-  a.s0 = search[0];
-  a.s1 = search[1];
-  a.gx0 = gridx[0];
-  a.gx1 = gridx[1];
-  a.gy0 = gridy[0];
-  a.gy1 = gridy[1];
-  a.winsize = winsize;
-  a.step = step;
-  a.nx = nx;
-  a.ny = ny;
   a.x = (double*)ox.dev;
   a.y = (double*)oy.dev;
   a.u = (double*)ou.dev;
   a.v = (double*)ov.dev;
   a.phi = (double*)op.dev;
-  a.I1 = c->I1;
-  a.I2 = c->I2;
-  a.tot = c->iitot;
-  a.tile_scratch = tbytes ? c->tscratch : nullptr;
-  a.ev_start = a.ev_stop = nullptr;
-  a.left = c->qcount + kSearchLeft;
-  a.path = &c->search_path;
-  a.impl = c->search_impl;
-  a.chunk = c->search_chunk;
   a.list = (const int*)al.dev;
-  a.nlist = list ? (long long)n : 0;
-  if (c->autotune && !list) {
+  if (tune) {
     rc = tune_search(c, a);
     if (rc) return rc;
   }
@@ -666,8 +658,31 @@ static int tune_icgn(aldic_ctx* c, IcgnArgs& a, int wmax) {
   return ALDIC_OK;
 }
 
+static std::string search_key(const SearchArgs& a) {
+  return shape_key("search", {a.M, a.N, a.winsize, a.step, a.s0, a.s1, a.nx, a.ny});
+}
+
+struct SearchCand {
+  int impl, chunk;
+  const char* name;
+};
+constexpr SearchCand kSearchCands[] = {{1, 24, "tile24"}, {1, 16, "tile16"}, {2, 0, "direct"}, {0, 0, "by_size"}};
+
+// Scratch of the shape's winner, or before it is known of every candidate.
+static size_t tune_search_bytes(aldic_ctx* c, SearchArgs a) {
+  const auto it = c->tuned.find(search_key(a));
+  size_t most = 0;
+  for (const SearchCand& cd : kSearchCands) {
+    a.impl = cd.impl;
+    a.chunk = cd.chunk;
+    if (it == c->tuned.end() || (it->second.a == cd.impl && it->second.b == cd.chunk))
+      most = std::max(most, search_choose(a));
+  }
+  return most;
+}
+
 static int tune_search(aldic_ctx* c, SearchArgs& a) {
-  const std::string key = shape_key("search", {a.M, a.N, a.winsize, a.step, a.s0, a.s1, a.nx, a.ny});
+  const std::string key = search_key(a);
   auto it = c->tuned.find(key);
   if (it == c->tuned.end()) {
     aldic_ctx::Tuned tn;
@@ -675,16 +690,12 @@ static int tune_search(aldic_ctx* c, SearchArgs& a) {
     std::vector<double> u0(n), v0(n), p0(n), u1(n), v1(n), p1(n);
     double best = 1e300;
     bool first = true;
-    struct Cand {
-      int impl, chunk;
-      const char* name;
-    };
-    const Cand cands[] = {{1, 24, "tile24"}, {1, 16, "tile16"}, {2, 0, "direct"}, {0, 0, "by_size"}};
-    for (const Cand& cd : cands) {
-      if (cd.impl == 1 && (!a.tile_scratch || !search_tile_available(a.step, a.winsize, cd.chunk))) continue;
+    for (const SearchCand& cd : kSearchCands) {
+      if (cd.impl == 1 && (!a.scratch || !search_tile_available(a.step, a.winsize, cd.chunk))) continue;
       SearchArgs b = a;
       b.impl = cd.impl;
       b.chunk = cd.chunk;
+      search_choose(b);
       b.ev_start = b.ev_stop = nullptr;
       double ms = 0;
       int rc = time_on_stream(c, [&] { return launch_search(b, c->stream); }, &ms);
@@ -716,6 +727,7 @@ static int tune_search(aldic_ctx* c, SearchArgs& a) {
   }
   a.impl = it->second.a;
   a.chunk = it->second.b;
+  search_choose(a);
   return ALDIC_OK;
 }
 

@@ -93,10 +93,12 @@ struct SearchArgs {
   double* I1;   // (M+1) x (N+1) integral images of g and g^2 (scratch)
   double* I2;
   double* tot;  // row-pass chunk totals (scratch, search_tot_bytes)
-  void* tile_scratch;  // shared-product search scratch (search_tile_bytes bytes), or null
+  void* scratch;         // of the transforms or the tile kernel (search_choose), or null
+  size_t scratch_bytes;  // its size: a kernel that needs more does not run
   cudaEvent_t ev_start, ev_stop;  // recorded around the correlation kernel when non-null
   int impl;   // 0: transforms, the shared-product tile kernel (where one exists for (step, w + 1)) or the
               // direct kernel, by size; 1: the tile kernel (direct without one); 2: the direct kernel
+  int fft = 0;  // transform size, 0 for the other kernels (search_choose)
   int chunk;  // tile kernel shift columns per pass: 16 or 24 (0: the shape's default)
   const int* list;  // grid subsets (i + j nx) to search, or null for the whole grid; with a list
                     // the direct kernel runs and writes the outputs compactly (slot k = list[k])
@@ -142,13 +144,13 @@ size_t search_tot_bytes(int M, int N);
 int launch_search(const SearchArgs& a, cudaStream_t st);
 int launch_search_direct(const SearchArgs& a, cudaStream_t st);  // the direct kernel alone
 bool search_direct_available(int winsize);
-// scratch of the tile kernel or the transforms, the larger; 0 where neither exists for the size
-size_t search_scratch_bytes(int M, int N, int winsize, int step, int nx, int ny, int s0, int s1);
+// Sets a.fft by the call's options and sizes; returns the scratch of the kernel that it takes (0: direct).
+size_t search_choose(SearchArgs& a);
 int launch_search_fft(const SearchArgs& a, cudaStream_t st);  // < 0: not for this call
 // Shared-product search (search_tile.cu): scratch size (0 when the step / window pair has
 // no tile kernel), and the launcher (returns the launch count, or -1 when not available).
 constexpr int kDefaultWarpCap = 8;   // default IcgnArgs / Sub1Args warp_cap
-size_t search_tile_bytes(int M, int N, int winsize, int step, int nx, int ny, int s0, int s1, int chunk = 0);
+size_t search_tile_bytes(const SearchArgs& a);
 int launch_search_tile(const SearchArgs& a, cudaStream_t st);
 struct CamPair {
   double P[24];  // P_L = K_L [I | 0] then P_R = K_R [R | T], each 3x4 row-major

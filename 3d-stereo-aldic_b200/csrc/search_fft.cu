@@ -581,7 +581,7 @@ static int transform_size(int winsize, int s0, int s1) {
   return 0;
 }
 
-// The transform size to take for a call, 0 for the other kernels.  The transforms' time goes with
+// The transform size that a call of implementation 0 takes, 0 for the other kernels.  The transforms' time goes with
 // n L^2, the tiles' with the waves of tiles and their products and shifts, the direct kernel's with
 // its shifts and template rounded up to its blocks; the factors (us) are fits to the measured times
 // of the three over windows of 21 to 49, steps of 8 to 32 and radii of 4 to 70, 55 us being what
@@ -591,7 +591,7 @@ static int transform_size(int winsize, int s0, int s1) {
 static int transform_for(const SearchArgs& a) {
   const int W1 = a.winsize + 1, nda = a.s0 + a.s1 + 3;
   const int L = transform_size(a.winsize, a.s0, a.s1);
-  if (a.impl != 0 || a.list || !a.tile_scratch || !L || a.M < W1 || a.N < W1 || !search_direct_available(a.winsize))
+  if (a.impl != 0 || a.list || !L || a.M < W1 || a.N < W1 || !search_direct_available(a.winsize))
     return 0;
   const double n = (double)a.nx * a.ny, fft = n * L * L * 5.5e-6, tile = search_tile_us(a);
   if (tile >= 0) return fft < tile ? L : 0;
@@ -599,24 +599,19 @@ static int transform_for(const SearchArgs& a) {
   return 55 + fft < direct ? L : 0;
 }
 
-size_t search_scratch_bytes(int M, int N, int winsize, int step, int nx, int ny, int s0, int s1) {
-  const size_t tile = search_tile_bytes(M, N, winsize, step, nx, ny, s0, s1);
-  const int L = transform_size(winsize, s0, s1);
-  if (!L || M < winsize + 1 || N < winsize + 1) return tile;
-  SearchArgs a{};
-  a.M = M;
-  a.N = N;
-  a.winsize = winsize;
-  a.nx = nx;
-  a.ny = ny;
-  a.s0 = s0;
-  a.s1 = s1;
-  return std::max(tile, search_tables_bytes(a, row_bytes(L, M) * row_columns(L, M, ny)));
+static size_t transform_bytes(const SearchArgs& a, int L) {
+  return search_tables_bytes(a, row_bytes(L, a.M) * row_columns(L, a.M, a.ny));
+}
+
+size_t search_choose(SearchArgs& a) {
+  a.fft = transform_for(a);
+  if (a.fft) return transform_bytes(a, a.fft);
+  return a.list || a.impl == 2 ? 0 : search_tile_bytes(a);
 }
 
 int launch_search_fft(const SearchArgs& a, cudaStream_t st) {
-  const int L = transform_for(a);
-  if (!L) return -1;
+  const int L = a.fft;
+  if (!L || !a.scratch || transform_bytes(a, L) > a.scratch_bytes) return -1;
   SearchTables t;
   const int launches = launch_search_tables(a, row_bytes(L, a.M) * row_columns(L, a.M, a.ny), &t, st);
   if (cudaMemsetAsync(a.left, 0, sizeof(int), st) != cudaSuccess) return -1;

@@ -16,7 +16,7 @@ struct SearchTables {
 };
 
 size_t search_tables_bytes(const SearchArgs& a, size_t row_bytes);
-// Fills the tables in a.tile_scratch (the last three are the caller's to write).  Returns the launches.
+// Fills the tables in a.scratch (the last three are the caller's to write).  Returns the launches.
 int launch_search_tables(const SearchArgs& a, size_t row_bytes, SearchTables* t, cudaStream_t st);
 void launch_search_refit(const SearchArgs& a, const SearchTables& t, cudaStream_t st);
 double search_tile_us(const SearchArgs& a);  // estimate of the tile kernel's time; < 0 without one

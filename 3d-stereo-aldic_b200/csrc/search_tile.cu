@@ -98,40 +98,30 @@ struct TileScratch {
 
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-inline size_t scratch_layout(int M, int N, int W1, int nx, int ny, int nda, size_t row_bytes, char* base,
-                             TileScratch* sc) {
-  const size_t MW = (size_t)(M - W1 + 1), NW = (size_t)(N - W1 + 1), n = (size_t)nx * ny;
+// The layout of a call's scratch: the tile kernel's, or the transforms' (their map holds one float a
+// position, and row spectra take the place of the excluded columns' products).
+inline size_t scratch_layout(const SearchArgs& a, bool fft, size_t row_bytes, TileScratch* sc) {
+  const size_t W1 = a.winsize + 1, MW = a.M - W1 + 1, NW = a.N - W1 + 1, n = (size_t)a.nx * a.ny, nda = a.s0 + a.s1 + 3;
   size_t off = 0;
-  auto take = [&](size_t bytes) {
-    char* p = base ? base + off : nullptr;
+  auto take = [&](auto** p, size_t bytes) {
+    if (sc) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>((char*)a.scratch + off);
     off += align256(bytes);
-    return p;
   };
-  char* pm = take(MW * NW * sizeof(float2));
-  char* pv = take(MW * NW * sizeof(double));
-  char* ph = take(MW * (size_t)ny * sizeof(double));
-  char* pp = take(n * sizeof(SubsetPrm));
-  char* pr = take(n * 4 * (size_t)nda * sizeof(float2));
-  char* pc = take(n * 2 * (size_t)nda * sizeof(float));
-  char* pb = take(n * sizeof(int));
-  char* pf = take(n * sizeof(float));  // >= the number of tiles
-  char* prr = take((size_t)nx * 8 * (size_t)(N + 1) * sizeof(double));
-  char* pvb = take(MW * ((NW + kVB - 1) / kVB) * sizeof(double));
-  char* pl = take(n * sizeof(int));
-  char* pw = take(row_bytes);
-  if (sc) {
-    sc->flist = (int*)pl;
-    sc->rows = pw;
-    sc->vb = (double*)pvb;
-    sc->rr = (double*)prr;
-    sc->cf = (float*)pf;
-    sc->map = (float2*)pm;
-    sc->V = (double*)pv;
-    sc->H = (double*)ph;
-    sc->prm = (SubsetPrm*)pp;
-    sc->ringv = (float2*)pr;
-    sc->cx = (float*)pc;
-    sc->best = (int*)pb;
+  TileScratch none, &s = sc ? *sc : none;
+  take(&s.map, MW * NW * (fft ? sizeof(float) : sizeof(float2)));
+  take(&s.V, MW * NW * sizeof(double));
+  take(&s.H, MW * a.ny * sizeof(double));
+  take(&s.prm, n * sizeof(SubsetPrm));
+  take(&s.ringv, n * 4 * nda * sizeof(float2));
+  take(&s.best, n * sizeof(int));
+  take(&s.rr, (size_t)a.nx * 8 * (a.N + 1) * sizeof(double));
+  take(&s.vb, MW * ((NW + kVB - 1) / kVB) * sizeof(double));
+  if (fft) {
+    take(&s.flist, n * sizeof(int));
+    take((char**)&s.rows, row_bytes);
+  } else {
+    take(&s.cx, n * 2 * nda * sizeof(float));
+    take(&s.cf, n * sizeof(float));  // >= the number of tiles
   }
   return off;
 }
@@ -1126,16 +1116,14 @@ bool search_tile_available(int step, int winsize, int chunk) {
   return tile_entry(step, winsize + 1, chunk, &e) && e.fits();
 }
 
-size_t search_tile_bytes(int M, int N, int winsize, int step, int nx, int ny, int s0, int s1, int chunk) {
-  const int W1 = winsize + 1;
+size_t search_tile_bytes(const SearchArgs& a) {
+  const int W1 = a.winsize + 1;
   TileEntry e;
-  if (!tile_entry(step, W1, chunk, &e) || M < W1 || N < W1 || nx <= 0 || ny <= 0) return 0;
-  return scratch_layout(M, N, W1, nx, ny, s0 + s1 + 3, 0, nullptr, nullptr);
+  if (!tile_entry(a.step, W1, a.chunk, &e) || a.M < W1 || a.N < W1 || a.nx <= 0 || a.ny <= 0) return 0;
+  return scratch_layout(a, false, 0, nullptr);
 }
 
-size_t search_tables_bytes(const SearchArgs& a, size_t row_bytes) {
-  return scratch_layout(a.M, a.N, a.winsize + 1, a.nx, a.ny, a.s0 + a.s1 + 3, row_bytes, nullptr, nullptr);
-}
+size_t search_tables_bytes(const SearchArgs& a, size_t row_bytes) { return scratch_layout(a, true, row_bytes, nullptr); }
 
 // The waves of tiles times their products and shifts: a fit to measured times, see search_fft.cu.
 double search_tile_us(const SearchArgs& a) {
@@ -1165,7 +1153,7 @@ static void launch_tables(const SearchArgs& a, const TileScratch& sc, bool zeros
 
 int launch_search_tables(const SearchArgs& a, size_t row_bytes, SearchTables* t, cudaStream_t st) {
   TileScratch sc;
-  scratch_layout(a.M, a.N, a.winsize + 1, a.nx, a.ny, a.s0 + a.s1 + 3, row_bytes, (char*)a.tile_scratch, &sc);
+  scratch_layout(a, true, row_bytes, &sc);
   launch_tables(a, sc, true, st);
   *t = SearchTables{(const float*)sc.map, sc.prm, sc.ringv, sc.best, sc.flist, sc.rows};
   return 4;
@@ -1179,11 +1167,12 @@ void launch_search_refit(const SearchArgs& a, const SearchTables& t, cudaStream_
 int launch_search_tile(const SearchArgs& a, cudaStream_t st) {
   const int W1 = a.winsize + 1;
   TileEntry e;
-  if (a.impl == 2 || !tile_entry(a.step, W1, a.chunk, &e) || !a.tile_scratch || a.M < W1 || a.N < W1 || !e.fits())
+  if (a.impl == 2 || !tile_entry(a.step, W1, a.chunk, &e) || !a.scratch || a.M < W1 || a.N < W1 || !e.fits() ||
+      search_tile_bytes(a) > a.scratch_bytes)
     return -1;
   const int nda = a.s0 + a.s1 + 3;
   TileScratch sc;
-  scratch_layout(a.M, a.N, W1, a.nx, a.ny, nda, 0, (char*)a.tile_scratch, &sc);
+  scratch_layout(a, false, 0, &sc);
   const long long n = (long long)a.nx * a.ny;
   launch_tables(a, sc, false, st);
   const int ntiles = ((a.nx + e.TI - 1) / e.TI) * ((a.ny + kTJ - 1) / kTJ);
