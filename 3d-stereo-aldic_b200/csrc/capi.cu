@@ -66,7 +66,7 @@ struct aldic_ctx {
   int staging = 0;      // ALDIC_OPT_STAGING
   int slow_nw = 2;      // ALDIC_OPT_SLOW_WARPS (FP32 slow pass, with ALDIC_OPT_SLOW_FP64 0)
   int slow_fp64 = 0;    // ALDIC_OPT_SLOW_FP64
-  int fp64_threads = 128;  // ALDIC_OPT_FP64_THREADS
+  int fp64_threads = kDefaultFp64Threads;  // ALDIC_OPT_FP64_THREADS
   int search_path = kSearchDirect;  // the kernel of the last search
   int search_impl = 0;  // ALDIC_OPT_SEARCH_IMPL
   int search_chunk = 0; // ALDIC_OPT_SEARCH_CHUNK

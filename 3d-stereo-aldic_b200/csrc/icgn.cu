@@ -31,7 +31,6 @@
 namespace aldic {
 
 constexpr int kNT = 128;    // threads per FP32 solve CTA
-constexpr int kNT64 = 512;  // threads per FP64 re-solve CTA
 constexpr int kSlowSubset = 2;   // queue-1 flag of a subset continued by the multi-warp pass
 constexpr int kMovedSubset = 4;  // queue-1 flag of a subset moved to the FP64 re-solve queue
 constexpr int kToFp64 = 5;       // hand-off code of the warp passes: re-solve in FP64
@@ -333,7 +332,8 @@ __device__ __forceinline__ double fp32_noise(double factor, int step, double bf,
 // from the initial guesses, so its decisions are the FP64 reference's.
 //
 // Both are bound by the latency of one subset (few subsets, a serial control thread), so the FP64
-// form, whose sums may be split any way, takes 512 threads a subset, and the FP32 form, whose
+// form, whose sums may be split any way, takes 512 threads a subset unless the caller sets another
+// number, and the FP32 form, whose
 // per-thread sums fix 128 threads, runs as many CTAs as fit.  The flood fills work on bit columns
 // (flood_bits), and the g-region fill of an iteration is skipped where no g is zero: its
 // result is the whole window then.  A plate with a hole (2048^2, winsize 32, 17 757 nodes):
@@ -1454,10 +1454,13 @@ int launch_icgn(const IcgnArgs& a, int wmax_enlarged, cudaStream_t st) {
   if ((a.band > 0 || a.slow_fp64) && a.variant != 2) {
     // FP64 re-solves: the subsets too close to call in FP32 and the long trajectories
     const size_t smem = solve_smem_bytes<true>(wmax_enlarged);
-    cudaFuncSetAttribute(icgn_solve_kernel<true, kNT64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int grid = occupancy_grid((const void*)icgn_solve_kernel<true, kNT64>, smem, kNT64);
+    const int nt = a.fp64_threads;
+    auto kern = nt == 128 ? icgn_solve_kernel<true, 128> : nt == 256 ? icgn_solve_kernel<true, 256>
+                                                                     : icgn_solve_kernel<true, 512>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int grid = occupancy_grid((const void*)kern, smem, nt);
     if ((long long)grid > a.n) grid = (int)a.n;
-    icgn_solve_kernel<true, kNT64><<<grid, kNT64, smem, st>>>(a, 2);
+    kern<<<grid, nt, smem, st>>>(a, 2);
     ++launches;
   }
   return launches;
