@@ -74,6 +74,7 @@ struct aldic_ctx {
   struct Tuned {
     std::string choice;                    // the winner, as JSON
     std::vector<std::pair<std::string, double>> ms;  // every candidate's time (ms; < 0: results differed)
+    std::string more;                      // further members of the report's entry
     int a = 0, b = 0, c = 0, d = 0;        // the winner's settings
   };
   std::map<std::string, Tuned> tuned;  // call-shape key -> winner
@@ -666,7 +667,8 @@ struct SearchCand {
   int impl, chunk;
   const char* name;
 };
-constexpr SearchCand kSearchCands[] = {{1, 24, "tile24"}, {1, 16, "tile16"}, {2, 0, "direct"}, {0, 0, "by_size"}};
+// The default choice by size first: an untuned call's results are what the others are held against.
+constexpr SearchCand kSearchCands[] = {{0, 0, "by_size"}, {1, 24, "tile24"}, {1, 16, "tile16"}, {2, 0, "direct"}};
 
 // Scratch of the shape's winner, or before it is known of every candidate.
 static size_t tune_search_bytes(aldic_ctx* c, SearchArgs a) {
@@ -690,6 +692,8 @@ static int tune_search(aldic_ctx* c, SearchArgs& a) {
     std::vector<double> u0(n), v0(n), p0(n), u1(n), v1(n), p1(n);
     double best = 1e300;
     bool first = true;
+    constexpr const char* kKernel[] = {"fft", "tile", "direct"};  // by kSearchFft ..
+    const char *name = "", *kernel = "";                          // the winner's
     for (const SearchCand& cd : kSearchCands) {
       if (cd.impl == 1 && (!a.scratch || !search_tile_available(a.step, a.winsize, cd.chunk))) continue;
       SearchArgs b = a;
@@ -700,28 +704,36 @@ static int tune_search(aldic_ctx* c, SearchArgs& a) {
       double ms = 0;
       int rc = time_on_stream(c, [&] { return launch_search(b, c->stream); }, &ms);
       if (rc) return rc;
+      if (cd.impl == 1 && *a.path != kSearchTile) continue;  // no memory for its tables
       CK(cudaMemcpyAsync((first ? u0 : u1).data(), b.u, n * 8, cudaMemcpyDeviceToHost, c->stream));
       CK(cudaMemcpyAsync((first ? v0 : v1).data(), b.v, n * 8, cudaMemcpyDeviceToHost, c->stream));
       CK(cudaMemcpyAsync((first ? p0 : p1).data(), b.phi, n * 8, cudaMemcpyDeviceToHost, c->stream));
       CK(cudaStreamSynchronize(c->stream));
       bool agree = true;
-      if (!first)  // u, v identical (both implementations match the FP64 search exactly), phi to 1e-5
+      if (!first)  // u, v identical (the implementations match the FP64 search), phi to 1e-5
         for (size_t i = 0; i < n && agree; ++i) {
           const bool un = std::isnan(u0[i]) && std::isnan(u1[i]), vn = std::isnan(v0[i]) && std::isnan(v1[i]);
           const bool pn = std::isnan(p0[i]) && std::isnan(p1[i]);
           agree = (un || u0[i] == u1[i]) && (vn || v0[i] == v1[i]) && (pn || std::fabs(p0[i] - p1[i]) <= 1e-5);
         }
       first = false;
-      if (cd.impl != 0) tn.ms.push_back({cd.name, agree ? ms : -ms});
+      if (cd.impl != 0) {
+        tn.ms.push_back({cd.name, agree ? ms : -ms});
+      } else {
+        char t[96];
+        std::snprintf(t, sizeof(t), ", \"by_size\": {\"kernel\": \"%s\", \"ms\": %.4f}", kKernel[*a.path], ms);
+        tn.more = t;
+      }
       if (agree && ms < best) {
         best = ms;
+        name = cd.name;
+        kernel = kKernel[*a.path];
         tn.a = cd.impl;
         tn.b = cd.chunk;
       }
     }
     char ch[160];
-    std::snprintf(ch, sizeof(ch), "{\"search\": \"%s\"}",
-                  tn.a == 0 ? "by_size" : tn.a == 2 ? "direct" : (tn.b == 16 ? "tile16" : "tile24"));
+    std::snprintf(ch, sizeof(ch), "{\"search\": \"%s\", \"kernel\": \"%s\"}", name, kernel);
     tn.choice = ch;
     it = c->tuned.emplace(key, tn).first;
   }
@@ -1565,7 +1577,7 @@ int aldic_tuning_report(aldic_ctx* c, char* buf, int64_t len) {
       r += t;
       f = false;
     }
-    r += "}}";
+    r += "}" + kv.second.more + "}";
   }
   r += "}";
   if ((int64_t)r.size() + 1 > len) return fail(c, ALDIC_ERR_ARG, "report needs %zu bytes", r.size() + 1);

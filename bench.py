@@ -1057,10 +1057,11 @@ def run_stereo(args, P, emit=True):
     pipe.icgn_events = None
     icgn_work = icgn_flops(pipe.buf["S"]["conv"].cpu().numpy(), P["w"])
     search_ms = prof_ms / max(prof_n, 1)
-    tuned = [t["choice"]["search"] for k, t in cS.tuning_report().items() if k.startswith("search")]
-    by_fft = all(t == "by_size" for t in tuned)  # the default choice, at this size the transforms
-    flops = (transform_flops if by_fft else tile_flops)(P["size"], P["size"], P["w"], P["step"], P["s_stereo"],
-                                                         P["s_stereo"])
+    # the kernel of the stereo search: the tuned one, or by size, which takes the transforms here
+    tuned = [t["choice"]["kernel"] for k, t in cS.tuning_report().items() if k.startswith("search")]
+    kernel = tuned[0] if tuned else "fft"
+    flops = {"fft": transform_flops, "tile": tile_flops, "direct": crop_flops}[kernel](
+        P["size"], P["size"], P["w"], P["step"], P["s_stereo"], P["s_stereo"])
     direct_flops = crop_flops(P["size"], P["size"], P["w"], P["step"], P["s_stereo"], P["s_stereo"])
     fp32_peak = measure_fp32_peak(torch, dev)
 
@@ -1116,16 +1117,18 @@ def run_stereo(args, P, emit=True):
                        "l2_flush": "inputs (4 x 8 MiB frames + 3 contexts of FP32 images/gradients/integral images) "
                                    "exceed the 126 MB L2 across a step", **P},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "fp32", "kernel": "fft_rows_kernel + ncc_fft_kernel (stereo integer search, transforms)"
-                         if by_fft else "ncc_tile_kernel (stereo integer search, shared products)",
+            "roofline": {"bound": "fp32",
+                         "kernel": {"fft": "fft_rows_kernel + ncc_fft_kernel (stereo integer search, transforms)",
+                                    "tile": "ncc_tile_kernel (stereo integer search, shared products)",
+                                    "direct": "ncc_search_kernel (stereo integer search, direct sums)"}[kernel],
                          "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                          "frac": achieved / fp32_peak if fp32_peak else None,
-                         "traffic": None if by_fft else TILE_TRAFFIC.get(args.workload), "traffic_unit": "bytes per launch",
+                         "traffic": TILE_TRAFFIC.get(args.workload) if kernel == "tile" else None, "traffic_unit": "bytes per launch",
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel "
                                            "at this workload (separate capture)",
                          "peak_source": "measured on this GPU: the faster of a scalar FFMA and a packed FFMA2 "
                                         "loop (MEASURED_PEAKS.json holds only HBM and bf16 tensor peaks)",
-                         "algorithmic_flops_per_launch": flops, "flops_counted": "5 L log2 L per transform" if by_fft else "products only (2 per f*g)",
+                         "algorithmic_flops_per_launch": flops, "flops_counted": "5 L log2 L per transform" if kernel == "fft" else "products only (2 per f*g)",
                          "direct_correlation_flops": direct_flops, "launch_ms": search_ms,
                          "launches_timed": prof_n},
             "roofline_icgn": {"bound": "fp32", "kernel": "stereo IC-GN call (classify, one-warp pass, slow-subset "

@@ -363,8 +363,9 @@ int aldic_measure_fp32_peak(aldic_ctx* ctx, double* tflops);
  *   ALDIC_OPT_AUTOTUNE       1: the first call of every call shape (IC-GN: variant, winsize, n
  *                            to a power of two; search: image, winsize, step, search region,
  *                            grid) times every candidate of the options above on its own
- *                            inputs, checks that all candidates' results agree, and keeps the
- *                            fastest for that shape (that call waits for the device);
+ *                            inputs, checks that they agree with the options' defaults (the
+ *                            search: the choice by size; IC-GN: the first candidate), and keeps
+ *                            the fastest that does for that shape (that call waits for the device);
  *                            aldic_tuning_report gives the choices and timings as JSON. */
 #define ALDIC_OPT_ITERATION_CAP 0
 #define ALDIC_OPT_STAGING 1
@@ -394,7 +395,9 @@ int aldic_set_option(aldic_ctx* ctx, int option, int value);
 int aldic_get_option(aldic_ctx* ctx, int option, int* value);
 /* The autotuner's choices so far as a JSON object {shape key: {"choice": {...}, "ms":
  * {candidate: time, ...}}} (a negative time marks a candidate whose results differed) into
- * buf (len bytes, NUL-terminated). */
+ * buf (len bytes, NUL-terminated).  A search's choice also names the kernel that runs ("fft",
+ * "tile" or "direct"), and its entry holds "by_size": {"kernel": ..., "ms": time}, the choice by
+ * size that the others are held against. */
 int aldic_tuning_report(aldic_ctx* ctx, char* buf, int64_t len);
 /* Margin around tol within which aldic_local_icgn re-decides an FP32 convergence test by an
  * FP64 re-solve of the subset: band x tol (default band 1e-3; a huge value re-solves every
