@@ -165,6 +165,9 @@ struct FftShape {
 };
 
 constexpr int kCand = 32;  // shifts whose order may be decided in FP64 before a subset goes to the list
+// FP64 values no further apart count as equal, and the first shift wins: the integral images' rounding
+// (45 ulp of the prefix sum of g^2) moves a value by 1e-11 on 2048 x 2048.
+constexpr double kSame = 1e-10;
 
 // Value of one shift in FP64, by a warp (in every lane).
 __device__ __noinline__ double shift_value(const SearchArgs& a, SubsetGeom s, int aa, int bb, SubsetPrm P) {
@@ -289,7 +292,8 @@ __global__ void __launch_bounds__(FftShape<L>::NT, FftShape<L>::MINB)
   using Sh = FftShape<L>;
   constexpr int B = Sh::B, NU = Sh::NU, NT = Sh::NT;
   extern __shared__ __align__(16) float2 S[];
-  __shared__ float s_lo[NT / 32], s_val[kCand];
+  __shared__ float s_lo[NT / 32];
+  __shared__ double s_val[kCand];
   __shared__ int s_ncand, s_cand[kCand];
   const int tid = threadIdx.x, lane = tid & 31;
   const int W1 = a.winsize + 1, NPT = (W1 + 1) / 2, nda = a.s0 + a.s1 + 3;
@@ -517,16 +521,21 @@ __global__ void __launch_bounds__(FftShape<L>::NT, FftShape<L>::MINB)
       for (int c = tid >> 5; c < nc; c += NT / 32) {
         const int lin = s_cand[c];
         const double v = shift_value(a, s, lin % s.na, lin / s.na, P);
-        if (lane == 0) s_val[c] = (float)v;
+        if (lane == 0) s_val[c] = v;
       }
       __syncthreads();
     }
     if (tid == 0) {
       int w = 0;
-      for (int c = 1; c < min(nc, kCand); ++c)
-        if (s_val[c] > s_val[w] || (s_val[c] == s_val[w] && s_cand[c] < s_cand[w])) w = c;
+      if (nc > 1 && nc <= kCand) {
+        double top = s_val[0];
+        for (int c = 1; c < nc; ++c) top = fmax(top, s_val[c]);
+        w = -1;
+        for (int c = 0; c < nc; ++c)
+          if (s_val[c] >= top - kSame && (w < 0 || s_cand[c] < s_cand[w])) w = c;
+      }
       // above 1: a variance sum that is all cancellation
-      const bool sure = P.gnorm < 1e15f && P.denT < 1e15 && m < 1.00001f && nc > 0 && nc <= kCand;
+      const bool sure = P.gnorm < 1e15f && P.denT < 1e15 && m < 1.00001f && nc > 0 && nc <= kCand && w >= 0;
       best[t] = sure ? s_cand[w] : -1;
       if (!sure) flist[atomicAdd(fcount, 1)] = (int)t;
     }
