@@ -1540,14 +1540,16 @@ int aldic_get_option(aldic_ctx* c, int option, int* value) {
     case ALDIC_OPT_FP64_THREADS:
       *value = c->fp64_threads;
       return ALDIC_OK;
-    case ALDIC_STAT_FP64_RESOLVES:
-    case ALDIC_STAT_STAGING_TIMEOUT: {
+    case ALDIC_STAT_STAGING_TIMEOUT:
+      *value = 0;
+      return ALDIC_OK;
+    case ALDIC_STAT_FP64_RESOLVES: {
       // counters the last aldic_local_icgn left in the context's queue block (waits for it)
       CK(cudaSetDevice(c->device));
       int q[16];
       CK(cudaMemcpyAsync(q, c->qcount, sizeof(q), cudaMemcpyDeviceToHost, c->stream));
       CK(cudaStreamSynchronize(c->stream));
-      *value = option == ALDIC_STAT_FP64_RESOLVES ? q[4] : q[8];
+      *value = q[4];
       return ALDIC_OK;
     }
     case ALDIC_STAT_SEARCH_LEFT:

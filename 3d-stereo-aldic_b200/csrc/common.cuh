@@ -163,105 +163,6 @@ __host__ __device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
 #endif
 }
 
-// Kahan-compensated accumulation (Kahan 1965), the compensation kept with the opposite sign:
-// the running total is s + k.  The caller forms y = x + k, fused into the term's own
-// operation (y = fma(a, b, k) for a product term), then
-//   t = s + y;  k = (s - t) + y;  s = t
-// (each operation rounded on its own: packed instructions or _rn intrinsics, never
-// contracted or reassociated).  The error of the total is bounded by ~2 ulp of sum |x|,
-// independent of the number of terms.
-__host__ __device__ __forceinline__ void kahan2(float2& s, float2& k, float2 y) {
-  const float2 t = fadd2(s, y);
-  k = fadd2(fsub2(s, t), y);
-  s = t;
-}
-
-__device__ __forceinline__ void kahan1(float& s, float& k, float y) {
-  const float t = __fadd_rn(s, y);
-  k = __fadd_rn(__fsub_rn(s, t), y);
-  s = t;
-}
-
-// Two stencils at once with packed FP32 pairs (.x: point a, .y: point b); each lane's
-// result is bit-identical to stencil16 at that point.
-__device__ __forceinline__ void bspline_weights_x2(float2 t, float2 w[4]) {
-  const float2 k = make_float2(1.0f / 56.0f, 1.0f / 56.0f);
-  w[0] = fmul2(k, fmul2(t, ffma2(t, ffma2(t, make_float2(-24.0f, -24.0f), make_float2(57.0f, 57.0f)),
-                                 make_float2(-33.0f, -33.0f))));
-  w[1] = fmul2(k, ffma2(t, ffma2(t, ffma2(t, make_float2(64.0f, 64.0f), make_float2(-117.0f, -117.0f)),
-                                 make_float2(-3.0f, -3.0f)),
-                        make_float2(56.0f, 56.0f)));
-  w[2] = fmul2(k, fmul2(t, ffma2(t, ffma2(t, make_float2(-64.0f, -64.0f), make_float2(75.0f, 75.0f)),
-                                 make_float2(45.0f, 45.0f))));
-  w[3] = fmul2(k, fmul2(t, ffma2(t, ffma2(t, make_float2(24.0f, 24.0f), make_float2(-15.0f, -15.0f)),
-                                 make_float2(-9.0f, -9.0f))));
-}
-
-__device__ __forceinline__ float2 stencil16_x2(const float* __restrict__ img, int M, int ia, int ib, float2 tr,
-                                               float2 tc) {
-  // ia, ib: element index of tap 0 (r0 + c0 M) of the two points
-  float2 wr[4], wc[4];
-  bspline_weights_x2(tr, wr);
-  bspline_weights_x2(tc, wc);
-  const float* pa = img + ia;
-  const float* pb = img + ib;
-  float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const float* qa = pa + c * M;
-    const float* qb = pb + c * M;
-    float2 col = fmul2(wr[0], make_float2(__ldg(qa), __ldg(qb)));
-    col = ffma2(wr[1], make_float2(__ldg(qa + 1), __ldg(qb + 1)), col);
-    col = ffma2(wr[2], make_float2(__ldg(qa + 2), __ldg(qb + 2)), col);
-    col = ffma2(wr[3], make_float2(__ldg(qa + 3), __ldg(qb + 3)), col);
-    acc = ffma2(wc[c], col, acc);
-  }
-  return acc;
-}
-
-// The two stencils of stencil16_x2 read from a staged shared-memory tile (column-major,
-// `pitch` rows); oa, ob are the tile offsets of tap 0.  Same operations in the same order,
-// so each lane's value is bit-identical to stencil16_x2 on the image.
-__device__ __forceinline__ float2 stencil16_x2_tile(const float* tile, int pitch, int oa, int ob, float2 tr,
-                                                    float2 tc) {
-  float2 wr[4], wc[4];
-  bspline_weights_x2(tr, wr);
-  bspline_weights_x2(tc, wc);
-  const float* pa = tile + oa;
-  const float* pb = tile + ob;
-  float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const float* qa = pa + c * pitch;
-    const float* qb = pb + c * pitch;
-    float2 col = fmul2(wr[0], make_float2(qa[0], qb[0]));
-    col = ffma2(wr[1], make_float2(qa[1], qb[1]), col);
-    col = ffma2(wr[2], make_float2(qa[2], qb[2]), col);
-    col = ffma2(wr[3], make_float2(qa[3], qb[3]), col);
-    acc = ffma2(wc[c], col, acc);
-  }
-  return acc;
-}
-
-// stencil16 on a staged tile (see stencil16_x2_tile); bit-identical to stencil16.
-__device__ __forceinline__ float stencil16_tile(const float* tile, int pitch, int o, float tr, float tc) {
-  float wr[4], wc[4];
-  bspline_weights(tr, wr);
-  bspline_weights(tc, wc);
-  const float* p = tile + o;
-  float acc = 0.f;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const float* q = p + c * pitch;
-    float col = wr[0] * q[0];
-    col = fmaf(wr[1], q[1], col);
-    col = fmaf(wr[2], q[2], col);
-    col = fmaf(wr[3], q[3], col);
-    acc = fmaf(wc[c], col, acc);
-  }
-  return acc;
-}
-
 // ---------------------------------------------------------------------------------
 // Reductions
 // ---------------------------------------------------------------------------------
@@ -301,26 +202,6 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double* scratch, doubl
 #pragma unroll
     for (int w = 0; w < NT / 32; ++w) s += scratch[w * K + threadIdx.x];
     out[threadIdx.x] = s;
-  }
-  __syncthreads();
-}
-
-// Block-wide FP64 sums of K per-thread FP32 partials, converting one value at a time so
-// that only the FP32 partials stay live (low register pressure for wide one-off sums).
-template <int K, int NT>
-__device__ __forceinline__ void block_sum_f32(float (&v)[K], double* scratch, double* out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const double s = warp_sum((double)v[k]);
-    if (lane == 0) scratch[warp * K + k] = s;
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < K; k += NT) {
-    double s = 0;
-#pragma unroll
-    for (int w = 0; w < NT / 32; ++w) s += scratch[w * K + k];
-    out[k] = s;
   }
   __syncthreads();
 }

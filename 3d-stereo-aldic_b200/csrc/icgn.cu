@@ -26,7 +26,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
-#include "tma.cuh"
+#include "tma.cuh"  // smem_u32
 
 namespace aldic {
 
@@ -1199,10 +1199,12 @@ static int occupancy_grid(const void* fn, size_t smem, int threads = kNT) {
   return sms * per_sm;
 }
 
-// The limits of the entry points (windows above them are refused, or not re-solved in FP64).
+// The limits of the entry points (windows above them are refused, or not re-solved in FP64).  They keep a
+// window below 102 rows and columns (icgn_smem_bytes(101) > 200 KB), within the bit columns' 128.
 size_t icgn_smem_bytes(int w) { return (size_t)(w + 1) * (w + 1) * (4 * sizeof(float) + 4); }
 size_t icgn_smem_bytes_f64(int w) { return (size_t)(w + 1) * (w + 1) * (sizeof(double) + 3 * sizeof(float) + 4); }
-// What icgn_solve_kernel takes (carve): never more than the limits above.
+// What icgn_solve_kernel takes (carve): below the limits above from windows of 16 on; smaller ones take a
+// few KB.
 template <bool F64>
 static size_t solve_smem_bytes(int w) {
   const size_t W1 = w + 1;
@@ -1212,7 +1214,7 @@ size_t sub1_smem_bytes(int wx, int wy) { return (size_t)(wx + 1) * (wy + 1) * (4
 
 
 // ================================================================================
-// Subpb1 for unmasked subsets: warp groups, as icgn_group_kernel
+// Subpb1 for unmasked subsets: warp groups, as icgn_tile_kernel
 // ================================================================================
 // Every subset without a mask region (either queue; any window size) is solved by a group of
 // NW warps with no shared image buffer and no block barrier; the FP64 control is replicated
@@ -1426,7 +1428,7 @@ __global__ void __launch_bounds__(kWT, 2) subpb1_group_kernel(Sub1Args a) {
 
 int launch_icgn(const IcgnArgs& a, int wmax_enlarged, cudaStream_t st) {
   int launches = 0;
-  // counts of buckets 0 and 1, the 2 work counters, the count of bucket 2, the staging flag
+  // counts of buckets 0 and 1, the 2 work counters, the count of bucket 2
   cudaMemsetAsync(a.qcount, 0, 16 * sizeof(int), st);
   const long long threads = a.n * 32;
   const int cb = 256;
@@ -1569,7 +1571,7 @@ int launch_subpb1(const Sub1Args& a, int wmax_x, int wmax_y, cudaStream_t st) {
     launches += 2;
   }
   {  // masked subsets and restarts: the general kernel on queue 1
-    // carve_sub1; never more than sub1_smem_bytes, the entry point's limit
+    // carve_sub1: below sub1_smem_bytes, the entry point's limit, from windows of 16 on
     const size_t smem = (size_t)(wmax_x + 1) * (wmax_y + 1) * 4 * sizeof(float) + 10 * (wmax_y + 1) * sizeof(uint64_t);
     cudaFuncSetAttribute(subpb1_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int grid = occupancy_grid((const void*)subpb1_solve_kernel, smem);

@@ -52,13 +52,18 @@ __device__ __forceinline__ f32x2_t psub(f32x2_t a, f32x2_t b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-// kahan2 of common.cuh
+// Kahan-compensated accumulation (Kahan 1965), the compensation kept with the opposite sign:
+// the running total is s + k.  The caller forms y = x + k, fused into the term's own
+// operation (y = fma(a, b, k) for a product term), then
+//   t = s + y;  k = (s - t) + y;  s = t
+// (each operation rounded on its own, never contracted or reassociated).  The error of the total is
+// bounded by ~2 ulp of sum |x|, independent of the number of terms.
 __device__ __forceinline__ void pkahan(f32x2_t& s, f32x2_t& k, f32x2_t y) {
   const f32x2_t t = padd(s, y);
   k = padd(psub(s, t), y);
   s = t;
 }
-// bspline_weights_x2 of common.cuh
+// bspline_weights of common.cuh for a pair of points
 __device__ __forceinline__ void pweights(f32x2_t t, f32x2_t w[4]) {
   const f32x2_t k = pk(1.0f / 56.0f, 1.0f / 56.0f);
   w[0] = pmul(k, pmul(t, pfma(t, pfma(t, pk(-24.0f, -24.0f), pk(57.0f, 57.0f)), pk(-33.0f, -33.0f))));
@@ -79,7 +84,7 @@ struct Taps {
   static __device__ __forceinline__ uint32_t at(uint32_t a, int e) { return a + 4u * (uint32_t)e; }
   static __device__ __forceinline__ const float* at(const float* a, int e) { return a + e; }
 };
-// stencil16_x2 of common.cuh on two tap-0 positions
+// stencil16 of common.cuh at two tap-0 positions
 template <bool SMEM>
 __device__ __forceinline__ f32x2_t pstencil(typename Taps<SMEM>::Ptr qa, typename Taps<SMEM>::Ptr qb, int pitch,
                                             f32x2_t tr, f32x2_t tc) {

@@ -139,7 +139,6 @@ int launch_net_patches(const FrameDev& fr, const double* coords, long long n, vo
 int net_predict(struct ::aldic_net* net, const FrameDev& fr, const double* coords_dev, long long n, double* U0,
                 double* F0);
 int launch_subpb1(const Sub1Args& a, int wmax_x, int wmax_y, cudaStream_t st);
-size_t search_smem_bytes(int winsize, int s0, int s1);
 size_t search_tot_bytes(int M, int N);
 int launch_search(const SearchArgs& a, cudaStream_t st);
 int launch_search_direct(const SearchArgs& a, cudaStream_t st);  // the direct kernel alone

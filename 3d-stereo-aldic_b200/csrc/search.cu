@@ -444,13 +444,6 @@ static int strip_columns(int w, int na_max, int nb_max, size_t budget) {
   return sb;
 }
 
-size_t search_smem_bytes(int winsize, int s0, int s1) {
-  const int na = crop_max(s0, s1);
-  const int sb = strip_columns(winsize, na, na, 200 * 1024);
-  const SearchLayout L = search_layout(winsize, na, sb);
-  return sizeof(float) * ((size_t)L.TR * L.W1 + (size_t)L.DR * L.DC);
-}
-
 size_t search_tot_bytes(int M, int N) {
   const size_t ntr = (M + kIT - 1) / kIT, ntc = (N + kIT - 1) / kIT;
   return (ntc * 2 * M + ntr * 2 * N + ntr * 2 * (N + 1)) * sizeof(double);

@@ -382,9 +382,9 @@ int aldic_measure_fp32_peak(aldic_ctx* ctx, double* tflops);
  *                            (default). */
 #define ALDIC_OPT_SLOW_FP64 6
 #define ALDIC_OPT_FP64_THREADS 7
-/* Read-only statistics of the last aldic_local_icgn (aldic_get_option; waits for the call):
- * subsets re-solved in FP64, and 1 if a staging load outlasted its wait (0: its loads do not wait
- * on a barrier). */
+/* Read-only (aldic_get_option): subsets that the last aldic_local_icgn re-solved in FP64 (waits
+ * for the call); whether a staging load outlasted its wait, always 0 (its loads wait on no
+ * barrier). */
 #define ALDIC_STAT_FP64_RESOLVES 100
 #define ALDIC_STAT_STAGING_TIMEOUT 101
 /* Read-only, of the last aldic_integer_search or aldic_integer_search_list (waits for it): the
