@@ -26,10 +26,23 @@ namespace aldic {
 
 namespace {
 
-// Error of a numerator over |T| |D| that the decision allows for.  FP32 transforms of 48 to 192 a side
-// are off by 0.3e-7 to 0.8e-7 of it on noise and speckles and by 2e-7 at worst on plane waves and ramps
-// (numpy's single-precision FFT against its double one); the bound leaves a factor of ten.
-constexpr float kFftErr = 32.f * 5.9604645e-8f;
+// Bound of a numerator's error over |T| |D|, in units of u = 2^-24, from the roundings of the passes
+// (first order; Higham, Accuracy and Stability of Numerical Algorithms, chapter 24).  A layer of complex
+// additions adds u in the 2-norm, a product with a rounded root 3 u (2 u by FMAs, Jeannerod et al. 2017,
+// and the root's own), a radix-3 step 5 u, a radix-5 step 8 u.  So one dimension of 16 B values costs
+// F = 7 + 3 + b with b = 5 (B = 3), 2, 8, 9, 6, 13, 12, 10 (B = 12), and
+//   D, two rows a transform:                  2 F + 1
+//   T, rows:                                  F + 1
+//      columns, n = W1 / B rows summed:       (8 + n / 4) sqrt(n) <= 48, then 3 + b
+//   the product:                              2
+//   the inverse, whose every output is at most the sum of |spectrum| / L^2 <= |T| |D| times the
+//   roundings on a path; two rows share one:  F + 2 (F + 1)
+//   T to FP32, 1 / (|T| L^2), 1 / sqrt:       7
+// An error of a spectrum in the 2-norm reaches a numerator at most times the other factor's norm
+// (Cauchy-Schwarz).  The sums are 136 (L = 64) to 192 (L = 144); 256 covers them with the second order.
+// Measured errors are far smaller (up to 3.4 u on plane waves and ramps); the bound is what makes the
+// choice of the maximum certain, and costs nothing on speckles, whose peaks stand clear of it.
+constexpr float kFftErr = 256.f * 5.9604645e-8f;
 
 // cos and sin of 2 pi k / 720: the roots of every radix below.
 struct Roots {
@@ -172,12 +185,22 @@ constexpr double kSame = 1e-10;
 // Value of one shift in FP64, by a warp (in every lane).
 __device__ __noinline__ double shift_value(const SearchArgs& a, SubsetGeom s, int aa, int bb, SubsetPrm P) {
   const int W1 = a.winsize + 1, lane = threadIdx.x & 31;
+  const int i0 = max(0, 1 - aa), i1 = min(W1, s.dr1 - s.dr0 + 2 - aa);  // the window's rows and columns inside D
+  const int j0 = max(0, 1 - bb), j1 = min(W1, s.dc1 - s.dc0 + 2 - bb);
+  const float* f = a.f + (s.ii - 1 + i0) + (size_t)(s.jj - 1 + j0) * a.M;
+  const float* g = a.g + (s.dr0 - 1 + aa + i0) + (size_t)(s.dc0 - 1 + bb + j0) * a.M;
+  const int R = i1 - i0, n = R * (j1 - j0), di = 32 % R, step = di + 32 / R * a.M;
+  int i = lane % R, k = i + lane / R * a.M;
   double num = 0.0;
-  for (int k = lane; k < W1 * W1; k += 32) {
-    const int i = k % W1, j = k / W1;
-    const int r = s.dr0 - 1 + aa + i, c = s.dc0 - 1 + bb + j;
-    if (r >= s.dr0 && r <= s.dr1 && c >= s.dc0 && c <= s.dc1)
-      num += ((double)a.f[(s.ii - 1 + i) + (size_t)(s.jj - 1 + j) * a.M] - P.fm) * (double)a.g[r + (size_t)c * a.M];
+#pragma unroll 8  // loads in flight
+  for (int p = lane; p < n; p += 32) {
+    num += ((double)__ldg(f + k) - P.fm) * (double)__ldg(g + k);
+    i += di;
+    k += step;
+    if (i >= R) {
+      i -= R;
+      k += a.M - R;
+    }
   }
   return ncc_at(a, s, aa, bb, warp_sum(num), P.denT, P.tolz);
 }
