@@ -536,16 +536,25 @@ __global__ void __launch_bounds__(kCgThreads) subpb2_cg_kernel(
   }
 }
 
-int subpb2_cg_blocks(long long n) {
-  int dev = 0, sms = 148, per_sm = 1;
+// CTAs that the two forms of the solve may have, all resident at once.  One node a thread: 3 an SM (168
+// registers), short barriers.  Several: as many as fit (7 an SM at 72 registers), for the loads in flight
+// (3 / 7 an SM, a solve of 38 iterations: 90 000 nodes 802 / 734 us, 490 000 3.87 / 2.62 ms, 1.68 M 13.2 /
+// 8.0 ms; five launches an iteration took 12.6 ms there).
+static void cg_limits(long long* one, long long* many) {
+  int dev = 0, sms = 148, per_one = 1, per_many = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, subpb2_cg_kernel<false>, kCgThreads, 0);
-  int one = 1;  // both forms must fit: they take the same grid
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, subpb2_cg_kernel<true>, kCgThreads, 0);
-  // up to 3 CTAs an SM: enough loads in flight for large meshes, and short barriers
-  const long long most = (long long)sms * std::max(1, std::min(std::min(per_sm, one), 3)), need = (n + kCgThreads - 1) / kCgThreads;
-  return (int)std::max(1LL, std::min(most, need));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_one, subpb2_cg_kernel<true>, kCgThreads, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_many, subpb2_cg_kernel<false>, kCgThreads, 0);
+  *one = (long long)sms * std::max(1, std::min(per_one, 3));
+  *many = (long long)sms * std::max(1, per_many);
+}
+
+int subpb2_cg_blocks(long long n) {
+  long long one, many;
+  cg_limits(&one, &many);
+  const long long need = (n + kCgThreads - 1) / kCgThreads;
+  return (int)std::max(1LL, std::min(need, need <= one ? one : many));
 }
 
 int subpb2_mesh_tables(long long n, long long n_el, const int* E, long long n_dir, const int* dir,
@@ -646,8 +655,10 @@ int launch_subpb2_cg(bool start, int iters, int blocks, long long n, const int* 
   const unsigned char* cnt = e.cnt;
   void* args[] = {&s, &iters, &n, &adj_ptr, &adj, &elem, &n_el, &Ke, &free_, &col, &val, &cnt, &D, &x, &r, &z, &p0,
                   &p1, &q, &parts, &tol2, &maxit, &sc};
-  const void* k = n <= (long long)blocks * kCgThreads ? (const void*)subpb2_cg_kernel<true>
-                                                      : (const void*)subpb2_cg_kernel<false>;
+  long long one, many;
+  cg_limits(&one, &many);
+  const void* k = blocks <= one && n <= blocks * (long long)kCgThreads ? (const void*)subpb2_cg_kernel<true>
+                                                                       : (const void*)subpb2_cg_kernel<false>;
   cudaLaunchCooperativeKernel(k, dim3((unsigned)blocks), dim3(kCgThreads), args, 0, st);
   return 1;
 }
