@@ -66,7 +66,7 @@ struct aldic_ctx {
   int staging = 0;      // ALDIC_OPT_STAGING
   int slow_nw = 2;      // ALDIC_OPT_SLOW_WARPS (FP32 slow pass, with ALDIC_OPT_SLOW_FP64 0)
   int slow_fp64 = 0;    // ALDIC_OPT_SLOW_FP64
-  int fp64_threads = kDefaultFp64Threads;  // ALDIC_OPT_FP64_THREADS
+  int fp64_threads = 0;  // ALDIC_OPT_FP64_THREADS
   int search_path = kSearchDirect;  // the kernel of the last search
   int search_impl = 0;  // ALDIC_OPT_SEARCH_IMPL
   int search_chunk = 0; // ALDIC_OPT_SEARCH_CHUNK
@@ -603,10 +603,11 @@ static int tune_icgn(aldic_ctx* c, IcgnArgs& a, int wmax) {
     double best = 1e300;
     bool first = true;
     // staging x warps per subset of the FP32 slow pass x threads per subset of the FP64
-    // re-solve x the warp pass's iteration cap
+    // re-solve (the window's and another number) x the warp pass's iteration cap
+    const int by_window = fp64_threads_for(a.winsize);
     for (int staging = 0; staging <= 1; ++staging)
       for (int snw : {2, 4})
-        for (int f64t : {128, 512})
+        for (int f64t : {by_window, by_window == 512 ? 256 : 512})
           for (int cap : {8, 16}) {
             IcgnArgs b = a;
             b.staging = staging;
@@ -1504,8 +1505,8 @@ int aldic_set_option(aldic_ctx* c, int option, int value) {
       c->slow_fp64 = value;
       return ALDIC_OK;
     case ALDIC_OPT_FP64_THREADS:
-      if (value != 128 && value != 256 && value != 512)
-        return fail(c, ALDIC_ERR_ARG, "FP64 threads must be 128, 256 or 512");
+      if (value != 0 && value != 128 && value != 256 && value != 512)
+        return fail(c, ALDIC_ERR_ARG, "FP64 threads must be 128, 256, 512, or 0 (by the window)");
       c->fp64_threads = value;
       return ALDIC_OK;
     default:

@@ -332,8 +332,7 @@ __device__ __forceinline__ double fp32_noise(double factor, int step, double bf,
 // from the initial guesses, so its decisions are the FP64 reference's.
 //
 // Both are bound by the latency of one subset (few subsets, a serial control thread), so the FP64
-// form, whose sums may be split any way, takes 512 threads a subset unless the caller sets another
-// number, and the FP32 form, whose
+// form, whose sums may be split any way, takes fp64_threads a subset, and the FP32 form, whose
 // per-thread sums fix 128 threads, runs as many CTAs as fit.  The flood fills work on bit columns
 // (flood_bits), and the g-region fill of an iteration is skipped where no g is zero: its
 // result is the whole window then.  A plate with a hole (2048^2, winsize 32, 17 757 nodes):
@@ -1426,6 +1425,13 @@ __global__ void __launch_bounds__(kWT, 2) subpb1_group_kernel(Sub1Args a) {
   }
 }
 
+// Threads a subset of the FP64 re-solve.  Small windows leave most of 512 threads idle, and with many
+// subsets in the queue that counts (128 / 256 / 512 threads, 12 000 subsets of which the band queues 5162 at
+// window 7, 175 at 21, 20 at 41: 3790 / 5359 / 8859, 1105 / 1086 / 1159, 699 / 697 / 690 us; all queued: 5147 /
+// 9550 / 18721, 1364 / 1902 / 3241, 1841 / 2068 / 3074).  Large windows gain from more threads (window 61, all
+// queued: 5685 / 4665 / 4411 us; 150 subsets 254 / 229 / 223).
+int fp64_threads_for(int winsize) { return winsize < 24 ? 128 : winsize < 52 ? 256 : 512; }
+
 int launch_icgn(const IcgnArgs& a, int wmax_enlarged, cudaStream_t st) {
   int launches = 0;
   // counts of buckets 0 and 1, the 2 work counters, the count of bucket 2
@@ -1456,7 +1462,7 @@ int launch_icgn(const IcgnArgs& a, int wmax_enlarged, cudaStream_t st) {
   if ((a.band > 0 || a.slow_fp64) && a.variant != 2) {
     // FP64 re-solves: the subsets too close to call in FP32 and the long trajectories
     const size_t smem = solve_smem_bytes<true>(wmax_enlarged);
-    const int nt = a.fp64_threads;
+    const int nt = a.fp64_threads ? a.fp64_threads : fp64_threads_for(a.winsize);
     auto kern = nt == 128 ? icgn_solve_kernel<true, 128> : nt == 256 ? icgn_solve_kernel<true, 256>
                                                                      : icgn_solve_kernel<true, 512>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

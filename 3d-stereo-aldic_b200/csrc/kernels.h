@@ -50,7 +50,7 @@ struct IcgnArgs {
   const double* F0;  // 4n initial displacement gradients [F11 F21 F12 F22] or null (the reference's 0)
   int slow_fp64; // 1: subsets still iterating after warp_cap are re-solved in FP64 (not the epipolar
                  // variant, whose slow subsets always take the FP32 multi-warp pass)
-  int fp64_threads;  // threads per subset of the FP64 re-solve kernel: 128, 256 or 512
+  int fp64_threads;  // threads per subset of the FP64 re-solve kernel: 128, 256, 512, or 0: by the window
   double* zncc;  // n or null (not epipolar): ZNCC of the window under the last evaluated warp,
                  // which is the returned [F U] for a converged subset (the acceptance test of a
                  // learned initial guess; sums of the last iteration, so no extra pass)
@@ -149,7 +149,7 @@ int launch_search_fft(const SearchArgs& a, cudaStream_t st);  // < 0: not for th
 // Shared-product search (search_tile.cu): scratch size (0 when the step / window pair has
 // no tile kernel), and the launcher (returns the launch count, or -1 when not available).
 constexpr int kDefaultWarpCap = 8;   // default IcgnArgs / Sub1Args warp_cap
-constexpr int kDefaultFp64Threads = 512;  // default IcgnArgs fp64_threads
+int fp64_threads_for(int winsize);  // what 0 takes: 128, 256 or 512
 size_t search_tile_bytes(const SearchArgs& a);
 int launch_search_tile(const SearchArgs& a, cudaStream_t st);
 struct CamPair {

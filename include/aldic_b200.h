@@ -378,8 +378,8 @@ int aldic_measure_fp32_peak(aldic_ctx* ctx, double* tflops);
  *                            FP32 multi-warp pass continues them (ALDIC_OPT_SLOW_WARPS warps
  *                            each), its convergence tests checked against the band like the
  *                            first pass's;
- *   ALDIC_OPT_FP64_THREADS   threads per subset of the FP64 re-solve: 128, 256 or 512
- *                            (default). */
+ *   ALDIC_OPT_FP64_THREADS   threads per subset of the FP64 re-solve: 128, 256, 512, or 0
+ *                            (default): by the window's size. */
 #define ALDIC_OPT_SLOW_FP64 6
 #define ALDIC_OPT_FP64_THREADS 7
 /* Read-only (aldic_get_option): subsets that the last aldic_local_icgn re-solved in FP64 (waits
