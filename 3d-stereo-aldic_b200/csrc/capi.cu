@@ -156,10 +156,11 @@ struct Arg {
   void* dev;
 };
 
-int stage(aldic_ctx* c, std::vector<Arg*> args) {
+// `extra`: bytes that the call takes from the arena after the staged arrays.
+int stage(aldic_ctx* c, std::vector<Arg*> args, size_t extra = 0) {
   c->arena.used = 0;
   c->back.clear();
-  size_t need = 0;
+  size_t need = extra ? extra + 256 : 0;
   for (Arg* a : args)
     if (a->user && !is_device_ptr(a->user) && a->bytes) need += ((a->bytes + 255) & ~size_t(255)) + 256;
   int rc = arena_reserve(c, need);
@@ -320,7 +321,7 @@ int aldic_load_image_raw(aldic_ctx* c, int slot, const void* img, int dtype, int
   const size_t npx = (size_t)M * N;
   Arg ai{img, npx * es, false, nullptr}, am{mask, mask ? npx * sizeof(double) : 0, false, nullptr};
   Arg ams{mean_std, mean_std ? 2 * sizeof(double) : 0, true, nullptr};
-  rc = stage(c, {&ai, &am, &ams});
+  rc = stage(c, {&ai, &am, &ams}, mask ? npx : 0);  // and the mask's bytes
   if (rc) return rc;
   int launched = 0;
   uint8_t* mk = nullptr;
