@@ -111,6 +111,7 @@ int fail(aldic_ctx* c, int code, const char* fmt, ...) {
 }
 
 int cuda_fail(aldic_ctx* c, cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here: a later call's check does not find it again
   return fail(c, ALDIC_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
@@ -135,6 +136,7 @@ int arena_reserve(aldic_ctx* c, size_t bytes) {
   CK(cudaStreamSynchronize(c->stream));
   if (c->arena.base) CK(cudaFree(c->arena.base));
   c->arena.base = nullptr;
+  c->arena.cap = 0;  // nothing is held if the allocation fails
   size_t cap = bytes + bytes / 2 + (1 << 20);
   CK(cudaMalloc(&c->arena.base, cap));
   c->arena.cap = cap;
@@ -199,11 +201,14 @@ int ensure_frame(aldic_ctx* c, int M, int N) {
   if (M < 8 || N < 8) return fail(c, ALDIC_ERR_ARG, "image must be at least 8 x 8 (got %d x %d)", M, N);
   if (c->M == M && c->N == N && c->img[0]) return ALDIC_OK;
   CK(cudaStreamSynchronize(c->stream));
-  for (int s = 0; s < 2; ++s)
-    if (c->img[s]) CK(cudaFree(c->img[s]));
-  if (c->mask) CK(cudaFree(c->mask));
-  if (c->gx) CK(cudaFree(c->gx));
-  if (c->gy) CK(cudaFree(c->gy));
+  // no frame is held until every buffer is there
+  c->M = c->N = 0;
+  c->img_ok[0] = c->img_ok[1] = c->has_mask = c->grad_ok = false;
+  void** bufs[] = {(void**)&c->img[0], (void**)&c->img[1], (void**)&c->mask, (void**)&c->gx, (void**)&c->gy};
+  for (void** b : bufs) {
+    if (*b) CK(cudaFree(*b));
+    *b = nullptr;
+  }
   const size_t npx = (size_t)M * N, ng = (size_t)(M - 6) * (N - 6);
   for (int s = 0; s < 2; ++s) CK(cudaMalloc(&c->img[s], npx * sizeof(float)));
   CK(cudaMalloc(&c->mask, npx));
@@ -1190,6 +1195,7 @@ int aldic_subpb2_set_mesh(aldic_ctx* c, int64_t n, int64_t n_el, const int32_t* 
     if (c->sp2) CK(cudaFree(c->sp2));
     c->sp2 = nullptr;
     c->sp2_cap = 0;
+    c->sp2_n = c->sp2_nel = 0;  // no mesh if the allocation fails
     CK(cudaMalloc(&c->sp2, bytes));
     c->sp2_cap = bytes;
   }

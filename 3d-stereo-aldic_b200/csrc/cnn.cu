@@ -988,6 +988,7 @@ namespace {
   do {                                                                            \
     cudaError_t e_ = (call);                                                      \
     if (e_ != cudaSuccess) {                                                      \
+      cudaGetLastError(); /* reported here, not again by a later check */         \
       net->err = std::string(#call) + ": " + cudaGetErrorString(e_);              \
       return ALDIC_ERR_CUDA;                                                      \
     }                                                                             \
