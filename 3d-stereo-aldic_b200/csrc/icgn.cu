@@ -1444,9 +1444,9 @@ int launch_icgn(const IcgnArgs& a, int wmax_enlarged, cudaStream_t st) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // nominal-window subsets without a mask region: one warp per subset, then the slow ones.
-  // Windows of which at least 4 CTAs' buffers fit an SM are staged in shared memory;
+  // Windows of which at least 7 CTAs' buffers fit an SM (up to 45 pixels) are staged in shared memory;
   // ALDIC_OPT_STAGING stages every window whose buffers fit.
-  const TileGeom geo = tile_geometry(a.winsize + 1, a.staging ? 1 : 4);
+  const TileGeom geo = tile_geometry(a.winsize + 1, a.staging ? 1 : 7);
   launches += launch_icgn_tile<1, false>(a, geo, sms, st);
   if (!a.slow_fp64 || a.variant == 2)  // the FP32 multi-warp pass continues the slow subsets
     launches += a.slow_nw == 4 ? launch_icgn_tile<4, true>(a, geo, sms, st)
