@@ -1444,9 +1444,11 @@ int launch_icgn(const IcgnArgs& a, int wmax_enlarged, cudaStream_t st) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // nominal-window subsets without a mask region: one warp per subset, then the slow ones.
-  // Windows of which at least 7 CTAs' buffers fit an SM (up to 45 pixels) are staged in shared memory;
-  // ALDIC_OPT_STAGING stages every window whose buffers fit.
-  const TileGeom geo = tile_geometry(a.winsize + 1, a.staging ? 1 : 7);
+  // Staged in shared memory by a rule on the window and n; ALDIC_OPT_STAGING stages every window whose
+  // buffers fit.
+  const int W1 = a.winsize + 1;
+  const bool staged = a.staging ? tile_ctas(W1) >= 1 : tile_staged(W1, a.n, sms);
+  const TileGeom geo = staged ? tile_geometry(W1) : TileGeom{0, 0, 0};
   launches += launch_icgn_tile<1, false>(a, geo, sms, st);
   if (!a.slow_fp64 || a.variant == 2)  // the FP32 multi-warp pass continues the slow subsets
     launches += a.slow_nw == 4 ? launch_icgn_tile<4, true>(a, geo, sms, st)

@@ -782,23 +782,33 @@ __global__ void __launch_bounds__(32 * NW * kTileGroups, 8 / NW) icgn_tile_kerne
   }
 }
 
-// The buffers of a CTA for windows of W1 x W1 pixels, or none (rows 0).  A column holds at least
-// W1 + 9 rows of both groups: the footprint of a small warp is W1 + 6, the rest is room for the
-// warp to move and stretch before the buffer is loaded again.  As many columns as fit without one
-// CTA less per SM.  Windows for which fewer than min_ctas CTAs fit an SM read the image: with so
-// few warps the shared-memory form is the slower one (20 000 subsets at 2048 x 2048, staged / from the
-// image: window 45, 8 CTAs, 1217 / 1351 us; 49, 6 CTAs, 1698 / 1518; 61, 4 CTAs, 2606 / 2116).
-inline TileGeom tile_geometry(int W1, int min_ctas) {
-  constexpr int kSmBytes = 227 * 1024, kCtaBytes = 5 * 1024;  // per CTA: static and reserved shared memory
+// The buffers of a CTA for windows of W1 x W1 pixels.  A column holds at least W1 + 9 rows of both
+// groups: the footprint of a small warp is W1 + 6, the rest is room for the warp to move and stretch
+// before the buffer is loaded again.
+constexpr int kSmBytes = 227 * 1024, kCtaBytes = 5 * 1024;  // per CTA: static and reserved shared memory
+inline int tile_pitch(int W1) { return W1 + (kTileGroups * (W1 + 9) - W1 + 31) / 32 * 32; }
+// CTAs an SM whose buffers fit its shared memory.
+inline int tile_ctas(int W1) {
+  const int fit = kSmBytes / (tile_pitch(W1) * (int)sizeof(float) * (W1 + 9) + kCtaBytes);
+  return fit < 8 ? fit : 8;
+}
+// As many columns as fit without one CTA less per SM.
+inline TileGeom tile_geometry(int W1) {
   TileGeom g;
-  g.pitch = W1 + (kTileGroups * (W1 + 9) - W1 + 31) / 32 * 32;
+  g.pitch = tile_pitch(W1);
   g.rows = g.pitch / kTileGroups;
-  const int col = g.pitch * (int)sizeof(float);
-  const int fit = kSmBytes / (col * (W1 + 9) + kCtaBytes), ctas = fit < 8 ? fit : 8;
-  if (ctas < min_ctas) return TileGeom{0, 0, 0};
-  g.cols = (kSmBytes / ctas - kCtaBytes) / col;
+  g.cols = (kSmBytes / tile_ctas(W1) - kCtaBytes) / (g.pitch * (int)sizeof(float));
   if (g.cols > W1 + 16) g.cols = W1 + 16;
   return g;
+}
+// Whether n windows are staged.  With 4 to 6 CTAs an SM (windows of 47 to 69) the pass has too few warps
+// when there are more subsets than run at once, and reading the image is faster (20 000 subsets at 2048 x
+// 2048, staged / from the image: window 45, 8 CTAs, 1217 / 1351 us; 49, 6 CTAs, 1698 / 1518; 61, 4 CTAs,
+// 2606 / 2116); of fewer subsets a warp's own time counts (window 61: 300 subsets 209 / 242 us, 1184, the
+// last that run at once, 238 / 281, 1500 417 / 357).
+inline bool tile_staged(int W1, long long n, int sms) {
+  const int ctas = tile_ctas(W1);
+  return ctas >= 7 || (ctas >= 4 && n <= (long long)kTileGroups * ctas * sms);
 }
 
 template <int NW, bool SLOW>

@@ -350,8 +350,8 @@ int aldic_measure_fp32_peak(aldic_ctx* ctx, double* tflops);
  * beyond FP32 summation order, and with the FP64 re-solve not at all in the codes):
  *   ALDIC_OPT_ITERATION_CAP  as aldic_set_iteration_cap (1..1000, default 8);
  *   ALDIC_OPT_STAGING        1: the IC-GN warp passes stage each subset's deformed window in
- *                            shared memory wherever its buffers fit; 0 (default): only where
- *                            enough of them fit an SM, else they gather from the image;
+ *                            shared memory wherever its buffers fit; 0 (default): where
+ *                            that is faster by the window and n, else from the image;
  *   ALDIC_OPT_SLOW_WARPS     warps per subset of the pass that continues the subsets still
  *                            iterating after the iteration cap: 2 (default) or 4;
  *   ALDIC_OPT_SEARCH_IMPL    aldic_integer_search: 0 (default) by size: correlation by FFTs,
