@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256) col2im_relu_kernel(const float* __restric
 // output maps (zero on the ring outside the crops): dZR = dC fD / 32 where fR > 0 (B, 10, 10,
 // 32), dZD = dC^T fR / 32 where fD > 0 (B, 18, 18, 32), BF16; dC (B, 8, 8, 81) FP32.
 //
-// One CTA per sample: dC and both feature crops (57 KB) in shared memory, lanes = channels, so
+// One CTA per sample: dC and both feature crops (61 696 bytes) in shared memory, lanes = channels, so
 // a dC entry is one broadcast for a warp.  A thread per output reading all three from L2 took
 // 149 us a batch of 256 for the two gradients; this form 50 us.  Each sum runs over the
 // offsets in the same order.
